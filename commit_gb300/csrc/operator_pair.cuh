@@ -53,6 +53,48 @@ struct DD2 {
     f2 s, e;
 };
 
+// double -> (h, l): h = z rounded to FP32, l = z - h in FP32.  By integer operations on the
+// bits: the conversion and subtraction instructions run at 2 lanes / clock / SM on this GPU
+// (measured; four of them per element were 1.2 ms of a 1M-streamline A').  Values outside
+// [2^-73, 2^126) take the instructions.
+__device__ __forceinline__ void split_bits(double z, float &h, float &l) {
+    const unsigned hi = (unsigned)__double2hiint(z), lo = (unsigned)__double2loint(z);
+    const unsigned a = hi & 0x7fffffffu, sg = hi & 0x80000000u;
+    if (a - 0x3b600000u < 0x47d00000u - 0x3b600000u) {
+        const unsigned lo2 = lo + 0x10000000u;
+        const unsigned a2 = a + (lo2 < lo ? 1u : 0u);
+        h = __uint_as_float(__funnelshift_l(lo2, a2 - 0x38000000u, 3) | sg);
+        const int r = (int)(lo2 & 0x1fffffffu) - 0x10000000;
+        l = __int2float_rn(r) * __uint_as_float((((a >> 20) - 948u) << 23) | sg);
+    } else if ((a | lo) == 0u) {
+        h = 0.f;
+        l = 0.f;
+    } else {
+        h = __double2float_rn(z);
+        l = __double2float_rn(z - (double)h);
+    }
+}
+
+// FP32 -> FP64 by integer operations, for normal values (zero gives 2^-127)
+__device__ __forceinline__ double widen_bits(float f) {
+    const unsigned b = __float_as_uint(f);
+    return __hiloint2double((int)((((b << 1) >> 4) + 0x38000000u) | (b & 0x80000000u)), (int)(b << 29));
+}
+
+__device__ __forceinline__ double widen(float f) {
+    const unsigned a = __float_as_uint(f) & 0x7fffffffu;
+    return a - 0x00800000u < 0x7f000000u ? widen_bits(f) : (double)f;
+}
+
+// s + e as a double (|e| is some units of the last place of s): one FP64 addition instead of
+// three FP64 instructions (see split_bits); from |s| >= 2^-40 on, 2^-127 for e = 0 is lost in it
+__device__ __forceinline__ double ff_join(float s, float e) {
+    const unsigned a = __float_as_uint(s) & 0x7fffffffu, c = __float_as_uint(e) & 0x7fffffffu;
+    if (a - 0x2b800000u < 0x7f800000u - 0x2b800000u && (c >= 0x00800000u || c == 0u)) return widen_bits(s) + widen_bits(e);
+    if ((a | c) == 0u) return 0.0;
+    return (double)s + (double)e;
+}
+
 // coefficient c = h + l split in FP32, broadcast to both halves, with -h precomputed
 struct Coef2 {
     f2 nh, h, l;
@@ -100,18 +142,18 @@ __device__ __forceinline__ void dd2_val(const DD2 &a, double &v0, double &v1) {
     float s0, s1, e0, e1;
     f2_unpack(a.s, s0, s1);
     f2_unpack(a.e, e0, e1);
-    v0 = (double)s0 + (double)e0;
-    v1 = (double)s1 + (double)e1;
+    v0 = ff_join(s0, e0);
+    v1 = ff_join(s1, e1);
 }
 
-// sum of the two halves (scalar float-float) as a double
-__device__ __forceinline__ double dd2_hsum(const DD2 &a) {
+// sum of the two halves (scalar float-float)
+__device__ __forceinline__ float2 dd2_hsum(const DD2 &a) {
     float s0, s1, e0, e1;
     f2_unpack(a.s, s0, s1);
     f2_unpack(a.e, e0, e1);
     ArFF::Acc x{s0, e0}, y{s1, e1};
     ArFF::add(x, y);
-    return ArFF::val(x);
+    return make_float2(x.s, x.e);
 }
 
 __device__ __forceinline__ DD2 dd2_shfl_xor(unsigned m, const DD2 &a, int lm, int w) {
@@ -214,10 +256,14 @@ __device__ __forceinline__ void forward_row_p(const Comps &C, const Group<LPV> &
                     const int64_t q = (int64_t)i * cm.xstride + col;
                     double xv = x[cm.xbase + q];
                     if (ex) xv = xv * pow2(-ex);
-                    double c = (double)l * xv;
-                    if (cm.eval) c *= (double)cm.eval[q];
-                    ch = __double2float_rn(c);
-                    cl = __double2float_rn(c - (double)ch);
+                    if (cm.eval) {
+                        const uint32_t ev = cm.eval[q];
+                        if (ev != 1u) xv *= (double)ev;
+                    }
+                    float xh, xl;
+                    split_bits(xv, xh, xl);
+                    ch = __fmul_rn(l, xh);
+                    cl = __fmaf_rn(l, xl, __fmaf_rn(l, xh, -ch));
                 }
                 // merged coefficient of each run (segmented inclusive scan, float-float)
                 int start = head;
@@ -241,8 +287,8 @@ __device__ __forceinline__ void forward_row_p(const Comps &C, const Group<LPV> &
                     const float tl = __shfl_sync(G.mask, cl, t, LPV);
                     const uint32_t rt = __shfl_sync(G.mask, row, t, LPV);
                     if (th != 0.f || tl != 0.f) {
-                        const Coef2 cf = coef2(th, tl);
                         const float *L = cm.lut + rt + base;
+                        const Coef2 cf = coef2(th, tl);
 #pragma unroll
                         for (int k = 0; k < NP; ++k) dd2_fma(acc[k], cf, f2_ldg(L + 2 * LPV * k));
                     }
@@ -312,11 +358,11 @@ struct PairBatch {
 };
 
 // <LUT row of item q, z> for the B items of a sub-batch (PairBatch); the total of item
-// q = sub / (LPV/B) ends in lane sub (butterfly reduce-scatter on packed accumulators,
-// halves combined at the end).
+// q = sub / (LPV/B) ends in lane sub (butterfly reduce-scatter on packed accumulators; the
+// caller adds the halves).
 template <int LPV, int NP, class RowFn>
-__device__ __forceinline__ double batch_dots_p(const Group<LPV> &G, const float *__restrict__ lut, RowFn row,
-                                               int cnt, const f2 (&zh)[NP], const f2 (&zl)[NP]) {
+__device__ __forceinline__ DD2 batch_dots_p(const Group<LPV> &G, const float *__restrict__ lut, RowFn row, int cnt,
+                                            const f2 (&zh)[NP], const f2 (&zl)[NP]) {
     constexpr int B = PairBatch<LPV, NP>::B;
     DD2 Pq[B];
     const int base = 2 * G.sub;
@@ -351,7 +397,7 @@ __device__ __forceinline__ double batch_dots_p(const Group<LPV> &G, const float 
     }
 #pragma unroll
     for (int m = LPV / PairBatch<LPV, NP>::B / 2; m >= 1; m /= 2) dd2_add(Pq[0], dd2_shfl_xor(G.mask, Pq[0], m, LPV));
-    return dd2_hsum(Pq[0]);
+    return Pq[0];
 }
 
 // A' pass 1 over all compartments.  Per batch, one dot product per run of equal
@@ -408,8 +454,11 @@ __global__ void __launch_bounds__(kBlock, MINB) k_adjoint_p(const OpDev P, const
             const unsigned h0 = abs_hi(z0), h1 = abs_hi(z1);
             zmax = h0 > zmax ? h0 : zmax;
             zmax = h1 > zmax ? h1 : zmax;
-            f2 unused;
-            split2(z0, z1, zh[k], zl[k], unused);
+            float s0, s1, t0, t1;
+            split_bits(z0, s0, t0);
+            split_bits(z1, s1, t1);
+            zh[k] = f2_pack(s0, s1);
+            zl[k] = f2_pack(t0, t1);
         }
         // range guard: a row outside float-float's range is split again, scaled (exact)
         const int ez = ff_exp_hi(group_max_u<LPV>(zmax, G.mask), P.lut_exp_adj);
@@ -461,14 +510,26 @@ __global__ void __launch_bounds__(kBlock, MINB) k_adjoint_p(const OpDev P, const
                         }
                         rest = mrem;
                         auto rowf = [&](int q) { return __shfl_sync(G.mask, row, src[q], LPV); };
-                        const double tot = batch_dots_p<LPV, NP>(G, cm.lut, rowf, cnt, zh, zl);
+                        const DD2 tot = batch_dots_p<LPV, NP>(G, cm.lut, rowf, cnt, zh, zl);
                         const int q = my_item - u0;
                         const bool mine = valid && q >= 0 && q < cnt;
-                        double t = __shfl_sync(G.mask, tot, mine ? q * SPAN : 0, LPV);
-                        if (ez) t = t * pow2(ez);
-                        if (mine) {
-                            if (cm.to_scratch) scratch[(size_t)i * P.n + j] = (double)l * t;
-                            else xout[cm.xbase + (size_t)i * cm.xstride + col] = t;
+                        const int from = mine ? q * SPAN : 0;
+                        if (cm.to_scratch) {
+                            const float2 hs = dd2_hsum(tot);
+                            const float ts = __shfl_sync(G.mask, hs.x, from, LPV);
+                            const float te = __shfl_sync(G.mask, hs.y, from, LPV);
+                            if (mine) {
+                                double t = ff_join(ts, te);
+                                if (ez) t = t * pow2(ez);
+                                scratch[(size_t)i * P.n + j] = widen(l) * t;
+                            }
+                        } else {  // single dot products: the last sum in FP64
+                            float s0, s1, e0, e1;
+                            f2_unpack(tot.s, s0, s1);
+                            f2_unpack(tot.e, e0, e1);
+                            double t = __shfl_sync(G.mask, ((double)s0 + (double)s1) + ((double)e0 + (double)e1), from, LPV);
+                            if (ez) t = t * pow2(ez);
+                            if (mine) xout[cm.xbase + (size_t)i * cm.xstride + col] = t;
                         }
                     }
                 }
