@@ -112,6 +112,8 @@ struct RhsPtrs {
     int active[kMaxRhs];            // 0: skip this vector (outputs untouched)
 };
 
+struct FfPlan;                      // shared-memory float-float products (smem_ff.cuh)
+
 }  // namespace cgb
 
 struct cgb_op {
@@ -186,6 +188,8 @@ struct cgb_op {
     float *tc_terms;                // adjoint IC terms in entry order
     float *tc_ax;                   // A x rows for the gradient (FISTA), on demand
     __nv_bfloat16 *tc_rows16;       // EC rows (nEC * ndirs) then ISO rows (nISO) as BF16, stride tc_np
+    cgb::FfPlan *ffp;               // run layout of the shared-memory products, built on first use
+    int ff_pinned;                  // a build or shape of the pair kernels was set: they run
     size_t bytes;
     int nsm;
     cgb::OpDev dev() const;
@@ -207,6 +211,15 @@ int launch_resnorm_grid(cgb_op *op, const double *x, const double *y, const doub
 int launch_gradient_grid(cgb_op *op, const double *x, const double *y, const double *sqw, double *grad,
                          double *partials, const double *ax_a, const double *ax_b, double ca, double cb,
                          cudaStream_t st, int arith, int *grid);
+// float-float products with the table in shared memory (smem_ff.cu)
+int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const double *yobs, const double *sqw,
+                 double *partials, cudaStream_t st, int *grid, int *ran);
+int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int *ran);
+int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, const double *sqw, const double *ax_a,
+                  const double *ax_b, double ca, double cb, double *partials, cudaStream_t st, int *grid,
+                  const double **z);
+int refresh_ff_plan(cgb_op *op);
+void free_ff_plan(cgb_op *op);
 int reduction_blocks(const cgb_op *op);
 void free_grad_state(cgb_op *op);
 // reduced-precision path (mixed.cu): FP32 rows, FP64 columns

@@ -291,6 +291,7 @@ int cgb::ensure_fib_acc(cgb_op *op, int slots) {
 static void free_op(cgb_op *op) {
     if (!op) return;
     free_grad_state(op);
+    free_ff_plan(op);
     void *ptrs[] = {op->lutIC, op->lutEC, op->lutISO, op->lutIC_p, op->lutEC_p, op->lutISO_p, op->lutIC_r, op->lutEC_r, op->lutISO_r, op->seg_l16, op->vox_ptr,
                     op->seg_f, op->eval, op->fib_ptr, op->fib_perm, op->fib_order, op->ec_ptr, op->ec_col, op->iso_ptr,
                     op->iso_col, op->seg_o, op->ec_o, op->seg_l, op->scratch, op->scratch32, op->partials,
@@ -577,6 +578,7 @@ int cgb_op_set_lut(cgb_op *op, const float *lutIC, const float *lutEC, const flo
                               cudaMemcpyDefault));
     }
     op->lut_r_kind = 0;  // reduced-precision copies are rebuilt on their next use
+    CGB_TRY(refresh_ff_plan(op));
     return update_lut_exponents(op);
 }
 
@@ -585,6 +587,7 @@ int cgb_op_ff_shape(cgb_op *op, int set, int *fwd, int *adj) {
     if (set >= 0) {
         if (set > 2) return fail(CGB_ERR_INVALID, "shape must be 0 (tune), 1 (default) or 2 (a warp per voxel)");
         op->ff_shape[0] = op->ff_shape[1] = set;
+        op->ff_pinned = 1;
     }
     if (fwd) *fwd = op->ff_shape[0];
     if (adj) *adj = op->ff_shape[1];

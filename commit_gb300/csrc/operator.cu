@@ -258,6 +258,19 @@ static int run_adjoint(cgb_op *op, const double *yin, int in_mode, const double 
     const bool mx = in_mode == 1 && !op->nolut;
     if (mx) CGB_TRY(measure_input(op, x, op->ncols, st));
     XScale guard(op, mx);
+    if (in_mode != 0 && arith == CGB_ARITH_FF && op->ff_variant != 0) {
+        // the shared-memory products take the residual as rows: one pass forms it, and the
+        // adjoint below is that of an ordinary row vector
+        const double *z = nullptr;
+        int g = 0;
+        CGB_TRY(residual_smem(op, in_mode, x, yobs, sqw, ax_a, ax_b, ca, cb, partials, st, &g, &z));
+        if (z) {
+            CGB_TRY(run_adjoint(op, z, 0, nullptr, nullptr, nullptr, nullptr, nullptr, 0.0, 0.0, xout, nullptr, st,
+                                arith, nullptr));
+            if (grid_out) *grid_out = g;
+            return CGB_OK;
+        }
+    }
     if (op->nolut) {
         const OpDev P = op->dev();
         int g = (op->nV + kBlock - 1) / kBlock;

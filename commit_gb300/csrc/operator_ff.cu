@@ -104,6 +104,9 @@ static int shaped(cgb_op *op, int which, int slot_default, int slot_wide, cudaSt
 
 int forward_ff(cgb_op *op, const double *x, double *y, double *ax, const double *yobs, const double *sqw,
                double *partials, cudaStream_t st, int *grid) {
+    int ran = 0;
+    CGB_TRY(forward_smem(op, x, y, ax, yobs, sqw, partials, st, grid, &ran));
+    if (ran) return CGB_OK;
     FwdPair L{op, x, y, ax, yobs, sqw, partials, st, grid};
     return shaped(op, 0, kOccFwdFF, kOccFwdFFWide, st, L);
 }
@@ -111,6 +114,11 @@ int forward_ff(cgb_op *op, const double *x, double *y, double *ax, const double 
 int adjoint_ff(cgb_op *op, const double *yin, int in_mode, const double *x, const double *yobs, const double *sqw,
                const double *ax_a, const double *ax_b, double ca, double cb, double *xout, double *partials,
                cudaStream_t st, int *grid) {
+    if (in_mode == 0) {
+        int ran = 0;
+        CGB_TRY(adjoint_smem(op, yin, xout, st, &ran));
+        if (ran) return CGB_OK;
+    }
     AdjPair L{op, yin, in_mode, x, yobs, sqw, ax_a, ax_b, ca, cb, xout, partials, st, grid};
     // the first A' call of any input mode chooses the shape, so a solve whose first A' is the
     // fused gradient does not change shape (and summation order) at its second

@@ -1,0 +1,1134 @@
+// Run layout, table images, kernels and launches of the shared-memory float-float products
+// (smem_ff.cuh).
+#include <cub/cub.cuh>
+
+#include <mutex>
+#include <vector>
+
+#include "operator_launch.cuh"
+#include "smem_ff.cuh"
+
+namespace cgb {
+namespace {
+
+using namespace detail;
+
+// ------------------------------------------------------------------ layout
+__global__ void k_run_heads(const uint16_t *__restrict__ o, int64_t n, uint32_t *__restrict__ head) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
+        head[j] = j == 0 || o[j] != o[j - 1];
+}
+
+__global__ void k_voxel_heads(const uint32_t *__restrict__ vox_ptr, int nV, uint32_t *__restrict__ head) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < nV && vox_ptr[v] < vox_ptr[v + 1]) head[vox_ptr[v]] = 1u;
+}
+
+// id[j] = runs that begin before segment j (exclusive scan of head)
+__global__ void k_run_fill(const uint32_t *__restrict__ head, const uint32_t *__restrict__ id,
+                           const uint16_t *__restrict__ o, int64_t n, uint32_t nruns, uint16_t *__restrict__ run_o,
+                           uint32_t *__restrict__ run_seg) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
+        if (head[j]) {
+            run_o[id[j]] = o[j];
+            run_seg[id[j]] = (uint32_t)j;
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) run_seg[nruns] = (uint32_t)n;
+}
+
+__global__ void k_run_ptr(const uint32_t *__restrict__ vox_ptr, const uint32_t *__restrict__ id, int nV, int64_t n,
+                          uint32_t nruns, uint32_t *__restrict__ run_ptr) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v <= nV) run_ptr[v] = v < nV && vox_ptr[v] < n ? id[vox_ptr[v]] : nruns;
+}
+
+// sort key of a voxel: its window, then its run count falling
+__global__ void k_perm_key(const uint32_t *__restrict__ run_ptr, int nV, uint64_t *__restrict__ key,
+                           uint32_t *__restrict__ val) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nV) return;
+    key[v] = ((uint64_t)(v / kVoxWindow) << 32) | (0xffffffffu - (run_ptr[v + 1] - run_ptr[v]));
+    val[v] = (uint32_t)v;
+}
+
+// first run of each voxel whose orientation is in range b or beyond
+__global__ void k_run_blk(const uint32_t *__restrict__ run_ptr, const uint16_t *__restrict__ run_o, int nV, int nb,
+                          int no, uint32_t *__restrict__ run_blk) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nV) return;
+    uint32_t lo = run_ptr[v];
+    const uint32_t end = run_ptr[v + 1];
+    for (int b = 0; b <= nb; ++b) {
+        uint32_t hi = end;
+        while (lo < hi) {
+            const uint32_t m = lo + (hi - lo) / 2;
+            if ((int)run_o[m] < b * no) lo = m + 1;
+            else hi = m;
+        }
+        run_blk[(size_t)b * nV + v] = b == nb ? end : lo;
+    }
+}
+
+// table images: A [chunk][row][fcs], A' [chunk][range][response][orientation][acs]
+__global__ void k_fwd_image(const float *__restrict__ lut, int rows, int nS, int nc, int width, int cs,
+                            float *__restrict__ img) {
+    const int64_t total = (int64_t)nc * rows * cs;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(q % cs);
+        const int64_t t = q / cs;
+        const int r = (int)(t % rows), c = (int)(t / rows);
+        const int s = c * width + k;
+        img[q] = k < width && s < nS ? lut[(size_t)r * nS + s] : 0.f;
+    }
+}
+
+__global__ void k_adj_image(const float *__restrict__ lut, int nIC, int ndirs, int nS, int nc, int width, int nb, int no,
+                            int cs, float *__restrict__ img) {
+    const int64_t total = (int64_t)nc * nb * nIC * no * cs;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(q % cs);
+        int64_t t = q / cs;
+        const int o = (int)(t % no);
+        t /= no;
+        const int i = (int)(t % nIC);
+        t /= nIC;
+        const int b = (int)(t % nb), c = (int)(t / nb);
+        const int d = b * no + o, s = c * width + k;
+        img[q] = k < width && s < nS && d < ndirs ? lut[((size_t)i * ndirs + d) * nS + s] : 0.f;
+    }
+}
+
+__global__ void k_col_max(const float *__restrict__ lut, int rows, int nS, int padded, float *__restrict__ colmax) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= padded) return;
+    float m = 0.f;
+    if (s < nS)
+        for (int r = 0; r < rows; ++r) m = fmaxf(m, lut[(size_t)r * nS + s]);
+    colmax[s] = m;
+}
+
+// bit 0: a table entry is negative or not finite
+__global__ void k_table_flags(const float *__restrict__ lut, int64_t n, unsigned *__restrict__ flags) {
+    bool bad = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bad |= !(lut[i] >= 0.f && lut[i] <= 3.0e38f);
+    if (bad) atomicOr(flags, 1u);
+}
+
+__global__ void k_eval_flags(const uint32_t *__restrict__ eval, int64_t n, unsigned *__restrict__ flags) {
+    bool bad = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bad |= eval[i] != 1u;
+    if (bad) atomicOr(flags, 2u);
+}
+
+int grid_n(int64_t n) {
+    int64_t g = (n + 255) / 256;
+    return (int)(g < 1 ? 1 : (g > 8192 ? 8192 : g));
+}
+
+// ------------------------------------------------------------------ run coefficients
+// c[i][r] = sum over the run's segments of l * x[i*nF + f] * eval, in float-float; x scaled
+// by the range guard's power of two.  A thread takes kCoefRuns runs at once: the chain run ->
+// segment -> x is three dependent loads, and the x gathers hit L2.
+constexpr int kCoefRuns = 4;
+
+__device__ __forceinline__ void seg_coef(const OpDev &P, double xv, size_t q, float l, int ex, int eval_ones, float &h,
+                                         float &e) {
+    if (ex) xv = xv * pow2(-ex);
+    if (!eval_ones) {
+        const uint32_t ev = P.eval[q];
+        if (ev != 1u) xv *= (double)ev;
+    }
+    float xh, xl;
+    split_bits(xv, xh, xl);
+    h = __fmul_rn(l, xh);
+    e = __fmaf_rn(l, xl, __fmaf_rn(l, xh, -h));
+}
+
+__global__ void __launch_bounds__(256) k_run_coef(const OpDev P, const uint32_t *__restrict__ run_seg, int64_t nruns,
+                                                  const double *__restrict__ x, int eval_ones,
+                                                  float2 *__restrict__ coef) {
+    const int ex = ff_exp_x(P);
+    for (int64_t r0 = blockIdx.x * (256ll * kCoefRuns) + threadIdx.x; r0 < nruns;
+         r0 += (int64_t)gridDim.x * (256 * kCoefRuns)) {
+        uint32_t beg[kCoefRuns], end[kCoefRuns], f[kCoefRuns];
+        float l[kCoefRuns];
+#pragma unroll
+        for (int u = 0; u < kCoefRuns; ++u) {
+            const int64_t r = r0 + 256 * u < nruns ? r0 + 256 * u : nruns - 1;
+            beg[u] = run_seg[r];
+            end[u] = run_seg[r + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < kCoefRuns; ++u) {
+            f[u] = P.seg_f[beg[u]];
+            l[u] = P.seg_l[beg[u]];
+        }
+        for (int i = 0; i < P.nIC; ++i) {
+            double xv[kCoefRuns];
+#pragma unroll
+            for (int u = 0; u < kCoefRuns; ++u) xv[u] = x[(size_t)i * P.nF + f[u]];
+#pragma unroll
+            for (int u = 0; u < kCoefRuns; ++u) {
+                float ch, cl;
+                seg_coef(P, xv[u], (size_t)i * P.nF + f[u], l[u], ex, eval_ones, ch, cl);
+                for (uint32_t j = beg[u] + 1; j < end[u]; ++j) {
+                    const size_t q = (size_t)i * P.nF + P.seg_f[j];
+                    float h, e;
+                    seg_coef(P, x[q], q, P.seg_l[j], ex, eval_ones, h, e);
+                    ff_add(ch, cl, h, e);
+                }
+                const float h = __fadd_rn(ch, cl);
+                if (r0 + 256 * u < nruns)
+                    coef[(size_t)i * nruns + r0 + 256 * u] = make_float2(h, __fsub_rn(cl, __fsub_rn(h, ch)));
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------ A
+// 8 lanes own a voxel, lane `sub` the sample pairs sub + 8k, k < NP, of the block's chunk
+// (16 * NP samples).  Odd groups take the pairs of an even / odd k swapped, so the two groups
+// of a half-warp read the two halves of a 128-byte line and their shared-memory loads do
+// not conflict (rows are a multiple of 128 bytes apart).
+template <int NP>
+__global__ void __launch_bounds__(kFwdThreads, 1) k_fwd_smem(const __grid_constant__ SmFwdArgs A) {
+    constexpr int NE = (NP + 1) & ~1, CS = 16 * NE, W = 16 * NP, GPB = kFwdThreads / 8;
+    extern __shared__ __align__(16) float tab[];
+    const unsigned full = 0xffffffffu;
+    const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3, par = grp & 1;
+    const int chunk = blockIdx.x % A.nc, cta = blockIdx.x / A.nc, ncta = (gridDim.x - chunk + A.nc - 1) / A.nc;
+    const int rows = A.nIC * A.ndirs;
+    fill_table<kFwdThreads>(tab, A.img + (size_t)chunk * rows * CS, rows * CS);
+    const int s_base = chunk * W;
+    // pair of register k: kk(k); in a row, even and odd k have a base each
+    auto kk = [&](int k) { return (k ^ 1) < NP ? k ^ par : k; };
+    const float *tb = tab + 2 * sub, *tb0 = tb + 16 * par, *tb1 = tb - 16 * par;
+    auto pair = [&](unsigned row, int k) {
+        return *reinterpret_cast<const f2 *>(((k ^ 1) < NP ? (k & 1 ? tb1 : tb0) : tb) + row + 16 * k);
+    };
+    const int ex = A.xmax ? ff_exp_hi((unsigned)(*A.xmax >> 32), A.lut_exp) : 0;
+    const bool even = (A.nS & 1) == 0 && A.vec_ok;
+    double nrm = 0.0;
+    const int last = A.p1 - A.p0, stride = ncta * GPB;
+    // the voxel of the next step and its runs are fetched during this one
+    auto voxel = [&](int pos) {
+        int v = -1;
+        if (pos < last) v = (int)A.vperm[A.p0 + pos];
+        return v < A.v0 || v >= A.v1 ? -1 : v;
+    };
+    int v = voxel(cta * GPB + grp), vn = voxel(cta * GPB + grp + stride);
+    uint32_t rb = v >= 0 ? A.run_ptr[v] : 0u, re = v >= 0 ? A.run_ptr[v + 1] : 0u;
+    fill_wait();
+    for (int w = cta * GPB; w < last; w += stride) {
+        const uint32_t rbn = vn >= 0 ? A.run_ptr[vn] : 0u, ren = vn >= 0 ? A.run_ptr[vn + 1] : 0u;
+        const int vnn = voxel(w + grp + 2 * stride);
+        const uint32_t eb = v >= 0 && A.nEC ? A.ec_ptr[v] : 0u, ee = v >= 0 && A.nEC ? A.ec_ptr[v + 1] : 0u;
+        const uint32_t ib = v >= 0 && A.nISO ? A.iso_ptr[v] : 0u, ie = v >= 0 && A.nISO ? A.iso_ptr[v + 1] : 0u;
+        // largest coefficient and whether all are finite and >= 0
+        float cm = 0.f;
+        bool ok = true;
+        for (int i = 0; i < A.nIC; ++i)
+            for (uint32_t j = rb + sub; j < re; j += 8) {
+                const float h = A.coef[(size_t)i * A.nruns + j].x;
+                ok = ok && h >= 0.f && h <= 3.0e38f;
+                cm = fmaxf(cm, h);
+            }
+        __syncwarp();
+#pragma unroll
+        for (int d = 4; d; d >>= 1) cm = fmaxf(cm, __shfl_xor_sync(full, cm, d, 8));
+        ok = ((__ballot_sync(full, !ok) >> ((threadIdx.x & 31) & ~7)) & 0xffu) == 0u;
+        for (uint32_t j = rbn + 16 * sub; j < ren; j += 128) prefetch_l2(A.coef + j);
+        for (uint32_t j = rbn + 64 * sub; j < ren; j += 512) prefetch_l2(A.run_o + j);
+        const int mine = (int)(re - rb + 7) / 8;  // this voxel's batches; the warp runs the most of its four
+        int nb = max(mine, __shfl_xor_sync(full, mine, 8));
+        nb = max(nb, __shfl_xor_sync(full, nb, 16));
+        DD2 acc[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) dd2_zero(acc[k]);
+        unsigned biased = 0u;  // halves that carry the bias cm * colmax
+#pragma unroll 1
+        for (int i = 0; i < A.nIC; ++i) {
+            const float2 *cf = A.coef + (size_t)i * A.nruns;
+            uint32_t j = rb + sub;
+            float2 nc = make_float2(0.f, 0.f);
+            uint32_t no = 0;
+            if (j < re) {
+                nc = cf[j];
+                no = A.run_o[j];
+            }
+#pragma unroll 1
+            for (int it = 0; it < nb; ++it) {
+                const float2 c = nc;
+                const unsigned row = ((unsigned)(i * A.ndirs) + no) * (unsigned)CS;
+                j += 8;
+                nc = make_float2(0.f, 0.f);
+                no = 0;
+                if (j < re) {
+                    nc = cf[j];
+                    no = A.run_o[j];
+                }
+                const bool gen = !ok || (it == 0 && i == 0);  // general sum for this group's batch
+                const bool nz = c.x != 0.f || c.y != 0.f;
+                unsigned g = __ballot_sync(full, nz && gen), f = __ballot_sync(full, nz && !gen);
+                g |= g >> 16;
+                g = (g | g >> 8) & 0xffu;
+                f |= f >> 16;
+                f = (f | f >> 8) & 0xffu;
+                // zero coefficients add exactly nothing, so a group may sit out a step
+                if (g) {
+                    const float gx = gen ? c.x : 0.f, gy = gen ? c.y : 0.f;
+#pragma unroll 2
+                    for (int t = 0; t < 8; ++t) {
+                        if (!(g >> t & 1u)) continue;
+                        const float h = __shfl_sync(full, gx, t, 8), l = __shfl_sync(full, gy, t, 8);
+                        const unsigned r = __shfl_sync(full, row, t, 8);
+                        const f2 h2 = f2_pack(h, h), l2 = f2_pack(l, l);
+#pragma unroll
+                        for (int k = 0; k < NP; ++k)
+                            dd2_fma_any(acc[k], h2, l2, pair(r, k), A.zero);
+                    }
+                }
+                const float fx = gen ? 0.f : c.x, fy = gen ? 0.f : c.y;
+                if (f == 0xffu) {
+#pragma unroll 4
+                    for (int t = 0; t < 8; ++t) {
+                        const float h = __shfl_sync(full, fx, t, 8), l = __shfl_sync(full, fy, t, 8);
+                        const unsigned r = __shfl_sync(full, row, t, 8);
+                        const f2 h2 = f2_pack(h, h), l2 = f2_pack(l, l);
+#pragma unroll
+                        for (int k = 0; k < NP; ++k)
+                            dd2_fma_same(acc[k], h2, l2, pair(r, k));
+                    }
+                } else {
+                    while (f) {
+                        const int t = __ffs(f) - 1;
+                        f &= f - 1;
+                        const float h = __shfl_sync(full, fx, t, 8), l = __shfl_sync(full, fy, t, 8);
+                        const unsigned r = __shfl_sync(full, row, t, 8);
+                        const f2 h2 = f2_pack(h, h), l2 = f2_pack(l, l);
+#pragma unroll
+                        for (int k = 0; k < NP; ++k)
+                            dd2_fma_same(acc[k], h2, l2, pair(r, k));
+                    }
+                }
+                if (ok && i == 0 && it == 0 && (mine > 1 || A.nIC > 1)) {
+                    // from here on the sums must not be below a term: add the bound where they may be
+#pragma unroll
+                    for (int k = 0; k < NP; ++k) {
+                        float m0, m1, a0, a1;
+                        f2_unpack(f2_ldg(A.colmax + s_base + 2 * (sub + 8 * kk(k))), m0, m1);
+                        f2_unpack(acc[k].s, a0, a1);
+                        m0 = __fmul_rn(cm, m0);
+                        m1 = __fmul_rn(cm, m1);
+                        const bool b0 = a0 < m0, b1 = a1 < m1;
+                        biased |= (b0 ? 1u << (2 * k) : 0u) | (b1 ? 2u << (2 * k) : 0u);
+                        dd2_addf(acc[k], f2_pack(b0 ? m0 : 0.f, b1 ? m1 : 0.f));
+                    }
+                } else if (ok && it < mine) {
+#pragma unroll
+                    for (int k = 0; k < NP; ++k) {
+                        const f2 s = f2_add(acc[k].s, acc[k].e);
+                        acc[k].e = f2_add(acc[k].e, f2_sub(acc[k].s, s));
+                        acc[k].s = s;
+                    }
+                }
+            }
+        }
+        if (biased) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                float m0, m1;
+                f2_unpack(f2_ldg(A.colmax + s_base + 2 * (sub + 8 * kk(k))), m0, m1);
+                dd2_addf(acc[k], f2_pack(biased >> (2 * k) & 1u ? -__fmul_rn(cm, m0) : 0.f,
+                                         biased >> (2 * k) & 2u ? -__fmul_rn(cm, m1) : 0.f));
+            }
+        }
+        __syncwarp();
+        // EC and ISO elements, (element, response) by (element, response); rows from L1 / L2
+        {
+            const int te = (int)(ee - eb) * A.nEC, tt = te + (int)(ie - ib) * A.nISO;
+            int m = max(tt, __shfl_xor_sync(full, tt, 8));
+            m = max(m, __shfl_xor_sync(full, m, 16));
+#pragma unroll 1
+            for (int b = 0; b < m; b += 8) {
+                const int q = b + sub;
+                float h = 0.f, l = 0.f;
+                const float *row = A.lutISO;
+                if (q < tt) {
+                    double xv;
+                    if (q < te) {
+                        const uint32_t j = eb + q / A.nEC;
+                        const int i = q % A.nEC;
+                        row = A.lutEC + (size_t)((unsigned)(i * A.ndirs) + A.ec_o[j]) * A.nSp;
+                        xv = A.x[A.ec_base + i * A.nE + A.ec_col[j]];
+                    } else {
+                        const int i = (q - te) % A.nISO;
+                        row = A.lutISO + (size_t)i * A.nSp;
+                        xv = A.x[A.iso_base + i * A.nISOv + A.iso_col[ib + (q - te) / A.nISO]];
+                    }
+                    if (ex) xv = xv * pow2(-ex);
+                    split_bits(xv, h, l);
+                }
+                unsigned g = __ballot_sync(full, h != 0.f || l != 0.f);
+                g |= g >> 16;
+                g = (g | g >> 8) & 0xffu;
+#pragma unroll
+                for (int k = 0; k < NP; ++k) {
+                    const f2 s = f2_add(acc[k].s, acc[k].e);
+                    acc[k].e = f2_add(acc[k].e, f2_sub(acc[k].s, s));
+                    acc[k].s = s;
+                }
+                while (g) {
+                    const int t = __ffs(g) - 1;
+                    g &= g - 1;
+                    const Coef2 q = coef2(__shfl_sync(full, h, t, 8), __shfl_sync(full, l, t, 8));
+                    const float *L = reinterpret_cast<const float *>(
+                                         __shfl_sync(full, reinterpret_cast<unsigned long long>(row), t, 8)) +
+                                     s_base + 2 * sub;
+#pragma unroll
+                    for (int k = 0; k < NP; ++k)
+                        dd2_fma(acc[k], q, s_base + 2 * (sub + 8 * kk(k)) < A.nSp ? f2_ldg(L + 16 * kk(k)) : 0ull);
+                }
+            }
+        }
+        if (v >= 0) {
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                const int s = s_base + 2 * (sub + 8 * kk(k));
+                if (s >= A.nS) continue;
+                float s0, s1, e0, e1;
+                f2_unpack(acc[k].s, s0, s1);
+                f2_unpack(acc[k].e, e0, e1);
+                double a0 = ff_join(s0, e0), a1 = ff_join(s1, e1);
+                if (ex) {
+                    a0 = a0 * pow2(ex);
+                    a1 = a1 * pow2(ex);
+                }
+                const size_t idx = (size_t)v * A.nS + s;
+                const bool two = s + 1 < A.nS;
+                if (A.yout) {
+                    if (two && even) *reinterpret_cast<double2 *>(A.yout + idx) = make_double2(a0, a1);
+                    else { A.yout[idx] = a0; if (two) A.yout[idx + 1] = a1; }
+                }
+                if (A.axout) {
+                    if (two && even) *reinterpret_cast<double2 *>(A.axout + idx) = make_double2(a0, a1);
+                    else { A.axout[idx] = a0; if (two) A.axout[idx + 1] = a1; }
+                }
+                if (A.partials) {
+                    double r0 = A.yobs ? a0 - A.yobs[idx] : a0;
+                    if (A.sqw) r0 *= A.sqw[idx];
+                    nrm = fma(r0, r0, nrm);
+                    if (two) {
+                        double r1 = A.yobs ? a1 - A.yobs[idx + 1] : a1;
+                        if (A.sqw) r1 *= A.sqw[idx + 1];
+                        nrm = fma(r1, r1, nrm);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        v = vn;
+        vn = vnn;
+        rb = rbn;
+        re = ren;
+    }
+    if (A.partials) {
+        __shared__ double red[kFwdThreads / 32];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) nrm += __shfl_xor_sync(full, nrm, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = nrm;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+            for (int q = 0; q < kFwdThreads / 32; ++q) t += red[q];
+            A.partials[(size_t)blockIdx.x * kRedSlots] = t;
+        }
+    }
+}
+
+// ------------------------------------------------------------------ A'
+// 8 lanes own a voxel and hold the block's chunk of its input row as float-float pairs (pairs
+// laid out as in A); a batch of 8 runs is taken four at a time (butterfly reduce-scatter as
+// batch_dots_p).  With one chunk each lane writes the terms l * <L, z> of one run's segments;
+// with several the runs' parts go to `part`, and the warp that finishes its four voxels last
+// of the chunks adds them and writes the terms.  EC / ISO elements of four voxels are taken
+// by the blocks of one of the orientation ranges in turn.
+
+// first two levels of the butterfly on four float-float pairs: lane sub is left with item
+// sub / 2, summed over half of the lanes
+__device__ __forceinline__ void scatter4(DD2 (&P)[4], int sub) {
+    const unsigned full = 0xffffffffu;
+#pragma unroll
+    for (int h = 2, m = 4; h >= 1; h /= 2, m /= 2) {
+        const bool up = (sub & m) != 0;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            DD2 send, keep;
+            send.s = up ? P[j].s : P[j + h].s;
+            send.e = up ? P[j].e : P[j + h].e;
+            keep.s = up ? P[j + h].s : P[j].s;
+            keep.e = up ? P[j + h].e : P[j].e;
+            dd2_add(keep, dd2_shfl_xor(full, send, m, 8));
+            P[j] = keep;
+        }
+    }
+}
+
+template <int NP>
+__global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_constant__ SmAdjArgs A) {
+    constexpr int NE = (NP + 1) & ~1, CS = 16 * NE, W = 16 * NP, GPB = kAdjThreads / 8;
+    extern __shared__ __align__(16) float tab[];
+    const unsigned full = 0xffffffffu;
+    const int sub = threadIdx.x & 7, par = (threadIdx.x >> 3) & 1;
+    const int parts = A.nc * A.nb, part = blockIdx.x % parts, chunk = part / A.nb, blk = part % A.nb;
+    const int s_base = chunk * W;
+    fill_table<kAdjThreads>(tab, A.img + (size_t)part * A.nIC * A.no * CS, A.nIC * A.no * CS);
+    auto kk = [&](int k) { return (k ^ 1) < NP ? k ^ par : k; };
+    const float *tb = tab + 2 * sub, *tb0 = tb + 16 * par, *tb1 = tb - 16 * par;
+    auto pair = [&](unsigned row, int k) {
+        return *reinterpret_cast<const f2 *>(((k ^ 1) < NP ? (k & 1 ? tb1 : tb0) : tb) + row + 16 * k);
+    };
+    const bool even = (A.nS & 1) == 0 && A.vec_ok;
+    const int last = A.p1 - A.p0, stride = (int)(gridDim.x / parts) * GPB;
+    // the voxel of the next step, its first runs and its row are fetched during this one
+    auto voxel = [&](int pos) {
+        int v = -1;
+        if (pos < last) v = (int)A.vperm[A.p0 + pos];
+        return v < A.v0 || v >= A.v1 ? -1 : v;
+    };
+    const uint32_t *rb_of = A.run_blk + (size_t)blk * A.nV, *re_of = rb_of + A.nV;
+    const int first = (int)(blockIdx.x / parts) * GPB + (int)(threadIdx.x >> 3);
+    int v = voxel(first), vn = voxel(first + stride);
+    uint32_t rb = v >= 0 ? rb_of[v] : 0u, re = v >= 0 ? re_of[v] : 0u;
+    unsigned on = rb + sub < re ? A.run_o[rb + sub] : 0u;  // orientation of this lane's next run
+    fill_wait();
+    for (int w = first - (int)((threadIdx.x & 31) >> 3); w < last; w += stride) {  // w: the warp's first position
+        const uint32_t rbn = vn >= 0 ? rb_of[vn] : 0u, ren = vn >= 0 ? re_of[vn] : 0u;
+        const int vnn = voxel(w + (int)((threadIdx.x & 31) >> 3) + 2 * stride);
+        f2 zh[NP], zl[NP];
+        unsigned zmax = 0, neg = 0;
+        auto load = [&](int k, double &z0, double &z1) {
+            const int s = s_base + 2 * (sub + 8 * kk(k));
+            z0 = z1 = 0.0;
+            if (v >= 0 && s < A.nS) {
+                const double *p = A.z + (size_t)v * A.nS + s;
+                if (even) {
+                    const double2 t = *reinterpret_cast<const double2 *>(p);
+                    z0 = t.x;
+                    z1 = t.y;
+                } else {
+                    z0 = p[0];
+                    if (s + 1 < A.nS) z1 = p[1];
+                }
+            }
+        };
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            double z0, z1;
+            load(k, z0, z1);
+            zmax = max(zmax, max(abs_hi(z0), abs_hi(z1)));
+            neg |= (unsigned)(__double2hiint(z0) | __double2hiint(z1));
+            float h0, l0, h1, l1;
+            split_bits(z0, h0, l0);
+            split_bits(z1, h1, l1);
+            zh[k] = f2_pack(h0, h1);
+            zl[k] = f2_pack(l0, l1);
+        }
+        if (vn >= 0) {
+            const char *p = reinterpret_cast<const char *>(A.z + (size_t)vn * A.nS + s_base);
+            if (128 * sub < 8 * W && s_base + 16 * sub < A.nS) prefetch_l2(p + 128 * sub);
+            for (uint32_t j = rbn + 32 * sub; j < ren; j += 256) prefetch_l2(A.run_seg + j);
+            for (uint32_t j = rbn + 64 * sub; j < ren; j += 512) prefetch_l2(A.run_o + j);
+        }
+        // range guard: a chunk of a row outside float-float's range is split again, scaled (exact)
+        const int ez = ff_exp_hi(group_max_u<8>(zmax, full), A.lut_exp);
+        if (ez) {
+#pragma unroll 1
+            for (int k = 0; k < NP; ++k) {
+                double z0, z1;
+                load(k, z0, z1);
+                f2 h, l, unused;
+                split2(z0 * pow2(-ez), z1 * pow2(-ez), h, l, unused);
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+                    if (q == k) {
+                        zh[q] = h;
+                        zl[q] = l;
+                    }
+            }
+        }
+        // rows without a negative entry take the five-operation sums (file comment of
+        // smem_ff.cuh): the bias is a power of two just below this lane's largest term bound
+        const bool pos = ((__ballot_sync(full, (neg >> 31) != 0u) >> ((threadIdx.x & 31) & ~7)) & 0xffu) == 0u;
+        const bool any_pos = __any_sync(full, pos), any_mix = __any_sync(full, !pos);
+        f2 bias;
+        {
+            float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                float a0, a1;
+                f2_unpack(f2_mul(zh[k], f2_ldg(A.colmax + s_base + 2 * (sub + 8 * kk(k)))), a0, a1);
+                x0 = fmaxf(x0, a0);
+                x1 = fmaxf(x1, a1);
+            }
+            auto down = [](float b) { return __uint_as_float(__float_as_uint(b * 1.001f) & 0x7f800000u); };
+            bias = f2_pack(down(x0), down(x1));
+        }
+        int most = (int)(re - rb);
+        most = max(most, __shfl_xor_sync(full, most, 8));
+        most = max(most, __shfl_xor_sync(full, most, 16));
+        if (most == 0) on = rbn + sub < ren ? __ldg(A.run_o + rbn + sub) : 0u;
+#pragma unroll 1
+        for (int b = 0; b < most; b += 8) {
+            const uint32_t j = rb + b + sub;
+            const bool valid = j < re;
+            const unsigned o = valid ? on - (unsigned)(blk * A.no) : 0u;
+            const int cnt = min(most - b, 8);
+            const uint32_t jn = b + 8 < most ? j + 8 : rbn + sub;
+            on = jn < (b + 8 < most ? re : ren) ? __ldg(A.run_o + jn) : 0u;
+#pragma unroll 1
+            for (int i = 0; i < A.nIC; ++i) {
+                const unsigned row = ((unsigned)(i * A.no) + o) * (unsigned)CS;
+                float ds = 0.f, de = 0.f;
+#pragma unroll 1
+                for (int u = 0; u < cnt; u += 4) {
+                    // this lane's run is item src of the four
+                    const int src = sub - u;
+                    const bool me = src >= 0 && src < 4;
+                    DD2 P[4], M;
+                    if (any_pos) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const unsigned r = __shfl_sync(full, row, u + q, 8);
+                            P[q].s = bias;
+                            P[q].e = 0ull;
+#pragma unroll
+                            for (int k = 0; k < NP; ++k)
+                                dd2_fma_same(P[q], zh[k], zl[k], pair(r, k));
+                            // the bias is a power of two not above s: the difference is exact
+                            P[q].s = f2_sub(P[q].s, bias);
+                        }
+                        scatter4(P, sub);
+                        M = P[0];
+                    }
+                    if (any_mix) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const unsigned r = __shfl_sync(full, row, u + q, 8);
+                            dd2_zero(P[q]);
+#pragma unroll
+                            for (int k = 0; k < NP; ++k)
+                                dd2_fma_any(P[q], zh[k], zl[k], pair(r, k), A.zero);
+                        }
+                        scatter4(P, sub);
+                        if (!pos) M = P[0];
+                    }
+                    dd2_add(M, dd2_shfl_xor(full, M, 1, 8));
+                    float ts, te, s1, e1;
+                    f2_unpack(M.s, ts, s1);
+                    f2_unpack(M.e, te, e1);
+                    ff_add(ts, te, s1, e1);
+                    const float rs = __shfl_sync(full, ts, me ? src * 2 : 0, 8);
+                    const float rl = __shfl_sync(full, te, me ? src * 2 : 0, 8);
+                    if (me) {
+                        ds = rs;
+                        de = rl;
+                    }
+                }
+                if (valid) {
+                    double t = ff_join(ds, de);
+                    if (ez) t = t * pow2(ez);
+                    if (A.nc > 1) {
+                        A.part[((size_t)i * A.nruns + j) * A.nc + chunk] = t;
+                    } else {
+                        for (uint32_t g = A.run_seg[j]; g < A.run_seg[j + 1]; ++g)
+                            A.scratch[(size_t)i * A.n + g] = widen(A.seg_l[g]) * t;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        const unsigned tile = (unsigned)(A.p0 + w) / 4u;
+        const bool ends = tile % (unsigned)A.nb == (unsigned)blk;  // this range takes the voxels' EC / ISO elements
+        uint32_t eb = 0, ib = 0;
+        int te = 0, tt = 0;
+        if (ends && v >= 0) {
+            if (A.nEC) {
+                eb = A.ec_ptr[v];
+                te = (int)(A.ec_ptr[v + 1] - eb) * A.nEC;
+            }
+            tt = te;
+            if (A.nISO) {
+                ib = A.iso_ptr[v];
+                tt += (int)(A.iso_ptr[v + 1] - ib) * A.nISO;
+            }
+        }
+        // column of (element, response) q, from the first EC column on; its table row
+        auto column = [&](int q) -> int64_t {
+            if (q < te) return (int64_t)(q % A.nEC) * A.nE + A.ec_col[eb + q / A.nEC];
+            q -= te;
+            return A.iso_base - A.ec_base + (int64_t)(q % A.nISO) * A.nISOv + A.iso_col[ib + q / A.nISO];
+        };
+        int m = max(tt, __shfl_xor_sync(full, tt, 8));
+        m = max(m, __shfl_xor_sync(full, m, 16));
+#pragma unroll 1
+        for (int b = 0; b < m; b += 8) {
+            const int q0 = b + sub;
+            const float *row = A.lutISO;
+            int64_t col = -1;
+            if (q0 < tt) {
+                col = column(q0);
+                row = q0 < te ? A.lutEC + (size_t)((unsigned)(q0 % A.nEC * A.ndirs) + A.ec_o[eb + q0 / A.nEC]) * A.nSp
+                              : A.lutISO + (size_t)((q0 - te) % A.nISO) * A.nSp;
+            }
+            const int cnt = min(m - b, 8);
+            double mine = 0.0;
+#pragma unroll 1
+            for (int u = 0; u < cnt; ++u) {
+                const float *L = reinterpret_cast<const float *>(
+                                     __shfl_sync(full, reinterpret_cast<unsigned long long>(row), u, 8)) +
+                                 s_base + 2 * sub;
+                DD2 P;
+                dd2_zero(P);
+#pragma unroll
+                for (int k = 0; k < NP; ++k)
+                    dd2_fma_any(P, zh[k], zl[k], s_base + 2 * (sub + 8 * kk(k)) < A.nSp ? f2_ldg(L + 16 * kk(k)) : 0ull,
+                                A.zero);
+                dd2_add(P, dd2_shfl_xor(full, P, 4, 8));
+                dd2_add(P, dd2_shfl_xor(full, P, 2, 8));
+                // the last sums round at the size of the result: in FP64 for these single dots
+                float s0, s1, e0, e1;
+                f2_unpack(P.s, s0, s1);
+                f2_unpack(P.e, e0, e1);
+                double t = ((double)s0 + (double)s1) + ((double)e0 + (double)e1);
+                t += __shfl_xor_sync(full, t, 1, 8);
+                if (sub == u) mine = t;
+            }
+            if (ez) mine = mine * pow2(ez);
+            if (col >= 0) {
+                if (A.nc > 1) A.epart[col * A.nc + chunk] = mine;
+                else A.xout[A.ec_base + col] = mine;
+            }
+        }
+        if (A.nc > 1) {
+            // the last of the chunks to finish these four voxels adds the parts
+            __threadfence();
+            __syncwarp();
+            unsigned before = 0;
+            unsigned *cell = A.arrive + (size_t)tile * A.nb + blk;
+            if ((threadIdx.x & 31) == 0) before = atomicAdd(cell, 1u);
+            before = __shfl_sync(full, before, 0);
+            if (before + 1u == (unsigned)A.nc) {
+                if ((threadIdx.x & 31) == 0) *cell = 0u;
+                __threadfence();
+                constexpr int U = 4;  // runs in flight per lane
+                for (uint32_t j0 = rb + sub; j0 < re; j0 += 8 * U) {
+                    uint32_t sb[U], se[U];
+                    float l[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t j = min(j0 + 8 * u, re - 1);
+                        sb[u] = __ldg(A.run_seg + j);
+                        se[u] = j0 + 8 * u < re ? __ldg(A.run_seg + j + 1) : sb[u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) l[u] = __ldg(A.seg_l + sb[u]);
+                    for (int i = 0; i < A.nIC; ++i) {
+                        double t[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+                            t[u] = __ldcg(A.part + ((size_t)i * A.nruns + min(j0 + 8 * u, re - 1)) * A.nc);
+                        for (int c = 1; c < A.nc; ++c) {
+#pragma unroll
+                            for (int u = 0; u < U; ++u)
+                                t[u] += __ldcg(A.part + ((size_t)i * A.nruns + min(j0 + 8 * u, re - 1)) * A.nc + c);
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+                            for (uint32_t g = sb[u]; g < se[u]; ++g)
+                                A.scratch[(size_t)i * A.n + g] = widen(g == sb[u] ? l[u] : __ldg(A.seg_l + g)) * t[u];
+                    }
+                }
+                for (int q0 = sub; q0 < tt; q0 += 8) {
+                    const int64_t col = column(q0);
+                    double t = __ldcg(A.epart + col * A.nc);
+                    for (int c = 1; c < A.nc; ++c) t += __ldcg(A.epart + col * A.nc + c);
+                    A.xout[A.ec_base + col] = t;
+                }
+            }
+            __syncwarp();
+        }
+        v = vn;
+        vn = vnn;
+        rb = rbn;
+        re = ren;
+    }
+}
+
+// weighted residual z = sqw * r, r = sqw * (A x - yobs) with A x = ax_a (mode 1) or
+// ca*ax_a + cb*ax_b (mode 2), and the block sums of r^2 (ax_a may be z)
+__global__ void __launch_bounds__(kBlock) k_residual(int64_t n, int mode, const double *ax_a,
+                                                     const double *__restrict__ ax_b, double ca, double cb,
+                                                     const double *__restrict__ yobs, const double *__restrict__ sqw,
+                                                     double *z, double *__restrict__ partials) {
+    double nrm = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)kBlock + threadIdx.x; i < n; i += (int64_t)gridDim.x * kBlock) {
+        const double av = mode == 1 ? ax_a[i] : ax_combine(ca, ax_a[i], cb, ax_b[i]);
+        double r = av - yobs[i];
+        if (sqw) r *= sqw[i];
+        nrm = fma(r, r, nrm);
+        z[i] = sqw ? sqw[i] * r : r;
+    }
+    if (partials) block_sum_store(nrm, partials + (size_t)blockIdx.x * kRedSlots);
+}
+
+struct Buf {
+    void *p = nullptr;
+    ~Buf() {
+        if (p) cudaFree(p);
+    }
+    template <class T>
+    int get(T **out, size_t count) {
+        CGB_CUDA(cudaMalloc(&p, (count ? count : 1) * sizeof(T)));
+        *out = (T *)p;
+        return CGB_OK;
+    }
+};
+
+template <class T>
+int keep(cgb_op *op, T **p, size_t count) {
+    CGB_CUDA(cudaMalloc((void **)p, (count ? count : 1) * sizeof(T)));
+    op->bytes += (count ? count : 1) * sizeof(T);
+    return CGB_OK;
+}
+
+constexpr size_t kTableBytes = 224 << 10;  // of the 227 KB a block may have
+
+// sample chunks of A: the fewest whose table part fits, at most 6 pairs per lane
+bool fwd_shape(int rows, int nS, FfPlan *f) {
+    for (int nc = (nS + 95) / 96; nc <= 64; ++nc) {
+        const int np = (nS + 16 * nc - 1) / (16 * nc), ne = (np + 1) & ~1;
+        if ((size_t)rows * 16 * ne * sizeof(float) > kTableBytes) {
+            if (np <= 2) return false;
+            continue;
+        }
+        if (np * 16 * (nc - 1) >= nS) return false;
+        f->fnp = np;
+        f->fnc = nc;
+        f->fcs = 16 * ne;
+        return true;
+    }
+    return false;
+}
+
+// sample chunks and orientation ranges of A': the fewest parts, then the fewest chunks
+bool adj_shape(int nIC, int ndirs, int nS, FfPlan *f) {
+    int best = 17;
+    for (int nc = (nS + 95) / 96; nc <= 16; ++nc) {
+        const int np = (nS + 16 * nc - 1) / (16 * nc), cs = 16 * ((np + 1) & ~1);
+        if (np < 2 || np * 16 * (nc - 1) >= nS) break;
+        const int per = (int)(kTableBytes / sizeof(float)) / cs / nIC;  // orientations that fit
+        if (per < 1) continue;
+        const int nb = (ndirs + per - 1) / per;
+        if (nc * nb >= best) continue;
+        best = nc * nb;
+        f->anc = nc;
+        f->anp = np;
+        f->anb = nb;
+        f->ano = (ndirs + nb - 1) / nb;
+        f->acs = cs;
+    }
+    return best <= 16;
+}
+
+int build_images(cgb_op *op, FfPlan *f) {
+    const int rows = op->nIC * op->ndirs;
+    if (f->fimg)
+        k_fwd_image<<<grid_n((int64_t)f->fnc * rows * f->fcs), 256>>>(op->lutIC, rows, op->nS, f->fnc, 16 * f->fnp,
+                                                                     f->fcs, f->fimg);
+    if (f->aimg)
+        k_adj_image<<<grid_n((int64_t)f->anc * f->anb * op->nIC * f->ano * f->acs), 256>>>(
+            op->lutIC, op->nIC, op->ndirs, op->nS, f->anc, 16 * f->anp, f->anb, f->ano, f->acs, f->aimg);
+    const int padded = kMaxSamples + 128;
+    k_col_max<<<(padded + 63) / 64, 64>>>(op->lutIC, rows, op->nS, padded, f->colmax);
+    CGB_CUDA(cudaGetLastError());
+    return CGB_OK;
+}
+
+int build_plan(cgb_op *op, FfPlan *f) {
+    const int64_t n = op->n;
+    const int nV = op->nV;
+    const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f), as = adj_shape(op->nIC, op->ndirs, op->nS, f);
+    if (!fs && !as) return CGB_OK;
+    Buf bh, bi, bt, bk, bk2, bv, bf;
+    uint32_t *head, *id;
+    CGB_TRY(bh.get(&head, (size_t)n));
+    CGB_TRY(bi.get(&id, (size_t)n));
+    k_run_heads<<<grid_n(n), 256>>>(op->seg_o, n, head);
+    k_voxel_heads<<<(nV + 255) / 256, 256>>>(op->vox_ptr, nV, head);
+    uint64_t *key, *key2;
+    uint32_t *val;
+    unsigned *flags;
+    CGB_TRY(bk.get(&key, (size_t)nV));
+    CGB_TRY(bk2.get(&key2, (size_t)nV));
+    CGB_TRY(bv.get(&val, (size_t)nV));
+    CGB_TRY(bf.get(&flags, 1));
+    size_t b1 = 0, b2 = 0;
+    CGB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b1, head, id, (int)n));
+    CGB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, b2, key, key2, val, val, nV, 0, 64));
+    char *tmp;
+    CGB_TRY(bt.get(&tmp, b1 > b2 ? b1 : b2));
+    CGB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, b1, head, id, (int)n));
+    CGB_CUDA(cudaMemset(flags, 0, sizeof(unsigned)));
+    k_table_flags<<<grid_n((int64_t)op->nIC * op->ndirs * op->nS), 256>>>(
+        op->lutIC, (int64_t)op->nIC * op->ndirs * op->nS, flags);
+    k_eval_flags<<<grid_n((int64_t)op->nF * op->nIC), 256>>>(op->eval, (int64_t)op->nF * op->nIC, flags);
+    uint32_t lastid[2];
+    unsigned hf = 0;
+    CGB_CUDA(cudaMemcpy(&lastid[0], id + (n - 1), 4, cudaMemcpyDeviceToHost));
+    CGB_CUDA(cudaMemcpy(&lastid[1], head + (n - 1), 4, cudaMemcpyDeviceToHost));
+    CGB_CUDA(cudaMemcpy(&hf, flags, 4, cudaMemcpyDeviceToHost));
+    f->nruns = (int64_t)lastid[0] + lastid[1];
+    f->eval_ones = !(hf & 2u);
+    if (hf & 1u) return CGB_OK;  // a negative or non-finite table entry: the pair kernels
+    CGB_TRY(keep(op, &f->run_ptr, (size_t)nV + 1));
+    CGB_TRY(keep(op, &f->run_o, (size_t)f->nruns));
+    CGB_TRY(keep(op, &f->run_seg, (size_t)f->nruns + 1));
+    CGB_TRY(keep(op, &f->vperm, (size_t)nV));
+    CGB_TRY(keep(op, &f->colmax, (size_t)kMaxSamples + 128));
+    k_run_fill<<<grid_n(n), 256>>>(head, id, op->seg_o, n, (uint32_t)f->nruns, f->run_o, f->run_seg);
+    k_run_ptr<<<(nV + 256) / 256, 256>>>(op->vox_ptr, id, nV, n, (uint32_t)f->nruns, f->run_ptr);
+    k_perm_key<<<(nV + 255) / 256, 256>>>(f->run_ptr, nV, key, val);
+    CGB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, b2, key, key2, val, f->vperm, nV, 0, 64));
+    if (fs) {
+        CGB_TRY(keep(op, &f->fimg, (size_t)f->fnc * op->nIC * op->ndirs * f->fcs));
+        CGB_TRY(keep(op, &f->coef, (size_t)op->nIC * f->nruns));
+        CGB_CUDA(cudaEventCreateWithFlags(&f->done, cudaEventDisableTiming));
+    }
+    if (as) {
+        CGB_TRY(keep(op, &f->aimg, (size_t)f->anc * f->anb * op->nIC * f->ano * f->acs));
+        if (f->anc > 1) {
+            const size_t cells = 2 * ((size_t)nV / 4 + 1) * f->anb;
+            CGB_TRY(keep(op, &f->part, (size_t)op->nIC * f->nruns * f->anc));
+            CGB_TRY(keep(op, &f->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * f->anc));
+            CGB_TRY(keep(op, &f->arrive, cells));
+            CGB_CUDA(cudaMemset(f->arrive, 0, cells * sizeof(unsigned)));
+        }
+        CGB_TRY(keep(op, &f->run_blk, (size_t)(f->anb + 1) * nV));
+        k_run_blk<<<(nV + 255) / 256, 256>>>(f->run_ptr, f->run_o, nV, f->anb, f->ano, f->run_blk);
+    }
+    CGB_TRY(build_images(op, f));
+    CGB_CUDA(cudaDeviceSynchronize());
+    f->fwd_ok = fs;
+    f->adj_ok = as;
+    return CGB_OK;
+}
+
+bool dense(const cgb_op *op, double items) { return (double)op->n * op->nIC >= items * op->nV; }
+
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// perm positions that hold the voxels [v0, v1): whole windows
+void perm_range(const cgb_op *op, int &v0, int &v1, int &p0, int &p1) {
+    v0 = op->vr1 > 0 ? op->vr0 : 0;
+    v1 = op->vr1 > 0 ? op->vr1 : op->nV;
+    p0 = v0 / kVoxWindow * kVoxWindow;
+    p1 = (v1 + kVoxWindow - 1) / kVoxWindow * kVoxWindow;
+    if (p1 > op->nV) p1 = op->nV;
+}
+
+// blocks of a launch: one per SM, a whole number for every part of the table
+int sm_grid(const cgb_op *op, int parts, int voxels, int per_block) {
+    int g = op->nsm / parts;
+    const int need = (voxels + per_block - 1) / per_block;
+    if (need < g) g = need;
+    return parts * (g < 1 ? 1 : g);
+}
+
+template <class F, class A>
+int launch_sm(F kern, int grid, int threads, size_t smem, cudaStream_t st, const A &a) {
+    CGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, threads, smem, st>>>(a);
+    CGB_CUDA(cudaGetLastError());
+    return CGB_OK;
+}
+
+}  // namespace
+
+void free_ff_plan(cgb_op *op) {
+    FfPlan *f = op->ffp;
+    if (!f) return;
+    void *p[] = {f->run_ptr, f->run_o, f->run_seg, f->coef, f->vperm, f->fimg, f->colmax, f->aimg, f->run_blk,
+                 f->part, f->epart, f->arrive, f->zrow};
+    for (void *q : p)
+        if (q) cudaFree(q);
+    if (f->done) cudaEventDestroy(f->done);
+    delete f;
+    op->ffp = nullptr;
+}
+
+// the handle's plan if the shared-memory kernels are to run this product, else null
+static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
+    *out = nullptr;
+    if (op->ff_variant != 1 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
+    if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork || !dense(op, kSmemMinItems)) return CGB_OK;
+    if (!op->ffp) {
+        if (capturing(st)) return CGB_OK;
+        static std::mutex m;
+        std::lock_guard<std::mutex> g(m);
+        if (!op->ffp) {
+            FfPlan *f = new FfPlan();
+            memset((void *)f, 0, sizeof(*f));
+            op->ffp = f;
+            const int rc = build_plan(op, f);
+            if (rc != CGB_OK) {
+                free_ff_plan(op);
+                return rc;
+            }
+        }
+    }
+    *out = op->ffp;
+    return CGB_OK;
+}
+
+int refresh_ff_plan(cgb_op *op) {
+    if (!op->ffp) return CGB_OK;
+    // new table: the sign check may change the choice of kernels, so the plan is laid out anew
+    // only when it does
+    Buf bf;
+    unsigned *flags, hf = 0;
+    CGB_TRY(bf.get(&flags, 1));
+    CGB_CUDA(cudaMemset(flags, 0, sizeof(unsigned)));
+    const int64_t cells = (int64_t)op->nIC * op->ndirs * op->nS;
+    k_table_flags<<<grid_n(cells), 256>>>(op->lutIC, cells, flags);
+    CGB_CUDA(cudaMemcpy(&hf, flags, 4, cudaMemcpyDeviceToHost));
+    FfPlan *f = op->ffp;
+    if ((hf & 1u) || !f->run_ptr) {
+        free_ff_plan(op);
+        return CGB_OK;
+    }
+    return build_images(op, f);
+}
+
+// A x with the table in shared memory; *ran = 0 when the pair kernels are to do it
+int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const double *yobs, const double *sqw,
+                 double *partials, cudaStream_t st, int *grid, int *ran) {
+    *ran = 0;
+    FfPlan *f;
+    CGB_TRY(plan_for(op, st, &f));
+    if (!f || !f->fwd_ok || !dense(op, kSmemMinItems)) return CGB_OK;
+    const OpDev P = op->dev();
+    SmFwdArgs a;
+    memset(&a, 0, sizeof(a));
+    a.vperm = f->vperm; a.run_ptr = f->run_ptr; a.run_o = f->run_o; a.coef = f->coef; a.nruns = f->nruns;
+    a.img = f->fimg; a.colmax = f->colmax;
+    a.nIC = op->nIC; a.ndirs = op->ndirs; a.nS = op->nS; a.nc = f->fnc;
+    perm_range(op, a.v0, a.v1, a.p0, a.p1);
+    a.ec_ptr = op->ec_ptr; a.ec_col = op->ec_col; a.ec_o = op->ec_o; a.iso_ptr = op->iso_ptr; a.iso_col = op->iso_col;
+    a.lutEC = op->lutEC_p; a.lutISO = op->lutISO_p; a.nSp = op->nSp;
+    a.nEC = op->nE > 0 ? op->nEC : 0; a.nISO = op->nISOv > 0 ? op->nISO : 0;
+    a.ec_base = P.ec_base; a.iso_base = P.iso_base; a.nE = op->nE; a.nISOv = op->nISOv;
+    a.x = x; a.xmax = P.xmax; a.lut_exp = P.lut_exp_fwd;
+    a.yout = y; a.axout = ax; a.yobs = yobs; a.sqw = sqw; a.partials = partials;
+    a.vec_ok = ((uintptr_t)y % 16 == 0) && ((uintptr_t)ax % 16 == 0);
+    // the coefficients belong to the handle: a product on another stream waits for the last
+    // one (under capture the graph's own order applies)
+    const bool cap = capturing(st);
+    if (!cap && f->used && f->last != st) CGB_CUDA(cudaStreamWaitEvent(st, f->done, 0));
+    if (op->vr1 <= 0 || op->vr0 == 0)
+        k_run_coef<<<grid_n((f->nruns + kCoefRuns - 1) / kCoefRuns), 256, 0, st>>>(P, f->run_seg, f->nruns, x, f->eval_ones, f->coef);
+    CGB_CUDA(cudaGetLastError());
+    const int g = sm_grid(op, f->fnc, a.p1 - a.p0, kFwdThreads / 8);
+    const size_t smem = (size_t)op->nIC * op->ndirs * f->fcs * sizeof(float);
+    int rc = CGB_ERR_UNSUPPORTED;
+    switch (f->fnp) {
+        case 1: rc = launch_sm(k_fwd_smem<1>, g, kFwdThreads, smem, st, a); break;
+        case 2: rc = launch_sm(k_fwd_smem<2>, g, kFwdThreads, smem, st, a); break;
+        case 3: rc = launch_sm(k_fwd_smem<3>, g, kFwdThreads, smem, st, a); break;
+        case 4: rc = launch_sm(k_fwd_smem<4>, g, kFwdThreads, smem, st, a); break;
+        case 5: rc = launch_sm(k_fwd_smem<5>, g, kFwdThreads, smem, st, a); break;
+        case 6: rc = launch_sm(k_fwd_smem<6>, g, kFwdThreads, smem, st, a); break;
+    }
+    CGB_TRY(rc);
+    if (!cap) {
+        CGB_CUDA(cudaEventRecord(f->done, st));
+        f->last = st;
+        f->used = 1;
+    }
+    if (grid) *grid = g;
+    *ran = 1;
+    return CGB_OK;
+}
+
+// voxel pass of A' with the table in shared memory over the current voxel range
+int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int *ran) {
+    *ran = 0;
+    FfPlan *f;
+    CGB_TRY(plan_for(op, st, &f));
+    if (!f || !f->adj_ok || !dense(op, 3 + 9 * f->anc)) return CGB_OK;
+    const OpDev P = op->dev();
+    SmAdjArgs a;
+    memset(&a, 0, sizeof(a));
+    a.vperm = f->vperm; a.run_blk = f->run_blk; a.run_seg = f->run_seg; a.run_o = f->run_o; a.seg_l = op->seg_l;
+    a.n = op->n; a.nruns = f->nruns; a.img = f->aimg; a.colmax = f->colmax;
+    a.nIC = op->nIC; a.nS = op->nS; a.nV = op->nV; a.nc = f->anc; a.nb = f->anb; a.no = f->ano;
+    perm_range(op, a.v0, a.v1, a.p0, a.p1);
+    a.ec_ptr = op->ec_ptr; a.ec_col = op->ec_col; a.ec_o = op->ec_o; a.iso_ptr = op->iso_ptr; a.iso_col = op->iso_col;
+    a.lutEC = op->lutEC_p; a.lutISO = op->lutISO_p; a.nSp = op->nSp; a.ndirs = op->ndirs;
+    a.nEC = op->nE > 0 ? op->nEC : 0; a.nISO = op->nISOv > 0 ? op->nISO : 0;
+    a.ec_base = P.ec_base; a.iso_base = P.iso_base; a.nE = op->nE; a.nISOv = op->nISOv;
+    a.z = z; a.lut_exp = P.lut_exp_adj; a.vec_ok = (uintptr_t)z % 16 == 0;
+    a.scratch = op->scratch; a.xout = xout; a.part = f->part; a.epart = f->epart;
+    // launches on the two streams of the slab schedule may overlap and share the four voxels
+    // at a boundary: they take the two halves of the arrival counts in turn
+    a.arrive = f->arrive + (f->flip ? ((size_t)op->nV / 4 + 1) * f->anb : 0);
+    f->flip ^= 1;
+    const int g = sm_grid(op, f->anc * f->anb, a.p1 - a.p0, kAdjThreads / 8);
+    const size_t smem = (size_t)op->nIC * f->ano * f->acs * sizeof(float);
+    int rc = CGB_ERR_UNSUPPORTED;
+    switch (f->anp) {
+        case 2: rc = launch_sm(k_adj_smem<2>, g, kAdjThreads, smem, st, a); break;
+        case 3: rc = launch_sm(k_adj_smem<3>, g, kAdjThreads, smem, st, a); break;
+        case 4: rc = launch_sm(k_adj_smem<4>, g, kAdjThreads, smem, st, a); break;
+        case 5: rc = launch_sm(k_adj_smem<5>, g, kAdjThreads, smem, st, a); break;
+        case 6: rc = launch_sm(k_adj_smem<6>, g, kAdjThreads, smem, st, a); break;
+    }
+    CGB_TRY(rc);
+    *ran = 1;
+    return CGB_OK;
+}
+
+// z = the weighted residual of a gradient pass in the plan's row buffer (in_mode 1 computes
+// A x first); *z stays null when the pair kernels are to do the gradient
+int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, const double *sqw, const double *ax_a,
+                  const double *ax_b, double ca, double cb, double *partials, cudaStream_t st, int *grid,
+                  const double **z) {
+    *z = nullptr;
+    FfPlan *f;
+    CGB_TRY(plan_for(op, st, &f));
+    if (!f || !f->adj_ok || !f->fwd_ok || !dense(op, 3 + 9 * f->anc)) return CGB_OK;
+    if (!f->zrow) {
+        if (capturing(st)) return CGB_OK;
+        CGB_TRY(keep(op, &f->zrow, (size_t)op->nrows));
+    }
+    if (in_mode == 1) {
+        int ran = 0;
+        CGB_TRY(forward_smem(op, x, f->zrow, nullptr, nullptr, nullptr, nullptr, st, nullptr, &ran));
+        if (!ran) return CGB_OK;
+        ax_a = f->zrow;
+    }
+    int g = (int)((op->nrows + kBlock - 1) / kBlock);
+    if (g > op->nsm * 8) g = op->nsm * 8;
+    k_residual<<<g, kBlock, 0, st>>>(op->nrows, in_mode, ax_a, ax_b, ca, cb, yobs, sqw, f->zrow, partials);
+    CGB_CUDA(cudaGetLastError());
+    if (grid) *grid = g;
+    *z = f->zrow;
+    return CGB_OK;
+}
+
+}  // namespace cgb

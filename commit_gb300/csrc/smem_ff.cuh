@@ -1,0 +1,167 @@
+// Float-float A*x and A'*y with the IC response table resident in shared memory.
+//
+// The pair kernels of operator_pair.cuh gather a table row per (voxel, orientation) run from
+// L1 / L2: 0.6 MB of FP32 rows at 500 orientations and 288 samples do not fit one SM's L1, so
+// at 1M streamlines the gathers (115 GB per product) bound them together with the 11 FP32
+// operations per term.  Here a block keeps a part of the table in shared memory for the
+// whole launch and walks every voxel:
+//   A   the block holds a chunk of the samples for every orientation and computes these
+//       samples of every row (no partial results leave the block);
+//   A'  the block holds a chunk of the samples for a range of orientations (all of them when
+//       they fit) and computes these samples' part of the runs' dot products; the block that
+//       finishes a few voxels last adds their parts up, from L2.
+// The runs (segments of a voxel with one orientation) are laid out once per handle
+// (FfPlan); A first forms each run's coefficient sum(l * x * eval) in one pass.
+//
+// Arithmetic.  A term is added to a float-float accumulator (s, e) as
+//   s' = fma(c.h, L, s);  d = s - s';  r = fma(c.h, L, d);  r = fma(c.l, L, r);  e += r
+// five FP32 operations instead of eleven: d is exact and r is the term's rounding error
+// whenever |c.h * L| <= |s| and s does not cancel.  Both hold when every term has the
+// sign of s and s starts at a bound of the terms (the bias), which is removed afterwards:
+//   A   x >= 0 and table >= 0 (checked per voxel / per handle): the first 8 runs are added
+//       with the general two-sum, the bias tops s up to max(c) * max(column) where it is
+//       below, and s, e are renormalised every 8 terms;
+//   A'  the bias is the sum of the negative terms' bounds plus the largest one, per lane.
+// Voxels with a negative or non-finite coefficient use the general two-sum throughout.
+#pragma once
+#include "operator_pair.cuh"
+
+namespace cgb {
+
+// Run layout and table images of a handle (built on the first large float-float product)
+struct FfPlan {
+    int fwd_ok, adj_ok;          // kernels usable for this handle's shape and table
+    int64_t nruns;
+    uint32_t *run_ptr;           // [nV+1] runs of voxel v
+    uint16_t *run_o;             // [nruns] orientation
+    uint32_t *run_seg;           // [nruns+1] first segment
+    float2 *coef;                // [nIC * nruns] run coefficients (high, low word) of the current A
+    uint32_t *vperm;             // [nV] voxels, by falling run count within windows of kVoxWindow
+    int eval_ones;               // eval is 1 everywhere
+    // A: samples in fnc chunks of 16 * fnp, row stride fcs floats
+    int fnp, fnc, fcs;
+    float *fimg;                 // [fnc][nIC * ndirs][fcs]
+    float *colmax;               // [>= nS] largest table value per sample, zero beyond nS
+    // A': samples in anc chunks of 16 * anp, orientations in anb ranges of ano, row stride acs
+    int anp, anc, anb, ano, acs;
+    float *aimg;                 // [anc][anb][nIC * ano][acs]
+    uint32_t *run_blk;           // [anb + 1][nV] first run of the voxel in a range
+    double *part;                // [nIC * nruns][anc] parts of the runs' dot products (anc > 1)
+    double *epart;               // [EC and ISO columns][anc]
+    unsigned *arrive;            // [2][voxels / 4 * anb] parts finished per four voxels
+    int flip;                    // half of arrive of the last launch (two may overlap)
+    double *zrow;                // [nrows] weighted residual (FISTA gradient)
+    cudaEvent_t done;            // the last product that used coef has finished
+    cudaStream_t last;           // ... and its stream
+    int used;
+};
+
+constexpr int kVoxWindow = 4096;
+constexpr int kFwdThreads = 768, kAdjThreads = 768;  // one block per SM, 80 registers a thread
+// Where the shared-memory kernels take over from the pair kernels of operator_pair.cuh: a
+// product of at least kSmemMinWork terms (segments x responses x samples) with at least
+// kSmemMinItems (A) or 3 + 9 * chunks (A') segments x responses per voxel.  Measured, us, here /
+// pair kernels: A 38 / 29 at 8 M terms, 43 / 38 at 17 M, 50 / 58 at 26 M; 101 / 116 at 13 per
+// voxel, 351 / 318 at 10 and 56 / 52 at 5.  A' per voxel: one chunk 139 / 150 at 13 (66 samples),
+// two 337 / 299 at 8 and 270 / 367 at 27 (145 and 99 samples), three 3461 / 3354 at 20 and
+// 2155 / 2541 at 33 (288 samples).  Below the lines the table fill (160-190 KB per SM) and the
+// per-voxel steps, repeated for every chunk, cost more than the gathers from L2.
+constexpr double kSmemMinWork = 2e7;
+constexpr double kSmemMinItems = 12;
+
+namespace detail {
+
+// a += b (exact two-sum into the error word)
+__device__ __forceinline__ void dd2_addf(DD2 &a, f2 b) {
+    const f2 s = f2_add(a.s, b);
+    const f2 bb = f2_sub(s, a.s);
+    const f2 err = f2_add(f2_sub(a.s, f2_sub(s, bb)), f2_sub(b, bb));
+    a.e = f2_add(a.e, err);
+    a.s = s;
+}
+
+// a += (h + l) * L for any terms: the two-sum of dd2_fma on the rounded product, whose last
+// difference takes the product itself, so its rounding error comes along (9 operations).
+// `zero` is 0 from a kernel argument: ptxas fuses a packed mul.rn whose only use is an add.rn
+// (measured, also with -fmad=false), which would leave the product unrounded.
+__device__ __forceinline__ void dd2_fma_any(DD2 &a, f2 h, f2 l, f2 L, f2 zero) {
+    const f2 s = f2_add(a.s, f2_fma(h, L, zero));
+    const f2 nb = f2_sub(a.s, s);
+    f2 r = f2_fma(h, L, nb);
+    r = f2_fma(l, L, r);
+    const f2 q = f2_sub(a.s, f2_add(s, nb));
+    a.e = f2_add(a.e, f2_add(r, q));
+    a.s = s;
+}
+
+// a += (h + l) * L for terms that neither exceed nor cancel a.s (file comment)
+__device__ __forceinline__ void dd2_fma_same(DD2 &a, f2 h, f2 l, f2 L) {
+    const f2 s = f2_fma(h, L, a.s);
+    const f2 d = f2_sub(a.s, s);
+    f2 r = f2_fma(h, L, d);
+    r = f2_fma(l, L, r);
+    a.e = f2_add(a.e, r);
+    a.s = s;
+}
+
+__device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ull; }
+
+// copies n floats (a multiple of 4, 16-byte aligned) to shared memory with all threads
+template <int THREADS>
+__device__ __forceinline__ void fill_table(float *dst, const float *__restrict__ src, int n) {
+    const unsigned d0 = (unsigned)__cvta_generic_to_shared(dst);
+    for (int i = threadIdx.x * 4; i < n; i += THREADS * 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d0 + 4u * i), "l"(src + i));
+    asm volatile("cp.async.commit_group;");
+}
+__device__ __forceinline__ void fill_wait() {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+}
+
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+struct SmFwdArgs {
+    const uint32_t *vperm, *run_ptr;
+    const uint16_t *run_o;
+    const float2 *coef;
+    int64_t nruns;
+    const float *img, *colmax;
+    int nIC, ndirs, nS, nc, p0, p1, v0, v1;   // perm positions [p0, p1), voxels [v0, v1)
+    const uint32_t *ec_ptr, *ec_col, *iso_ptr, *iso_col;
+    const uint16_t *ec_o;
+    const float *lutEC, *lutISO;              // padded rows of stride nSp
+    int nSp, nEC, nISO;
+    int64_t ec_base, iso_base, nE, nISOv;
+    const double *x;
+    const unsigned long long *xmax;
+    int lut_exp;
+    double *yout, *axout;
+    const double *yobs, *sqw;
+    double *partials;
+    int vec_ok;
+    f2 zero;                                  // 0 (dd2_fma_any)
+};
+
+struct SmAdjArgs {
+    const uint32_t *vperm, *run_blk, *run_seg;
+    const uint16_t *run_o;
+    const float *seg_l;
+    int64_t n, nruns;
+    const float *img, *colmax;
+    int nIC, nS, nV, nc, nb, no, p0, p1, v0, v1;
+    const uint32_t *ec_ptr, *ec_col, *iso_ptr, *iso_col;
+    const uint16_t *ec_o;
+    const float *lutEC, *lutISO;
+    int nSp, ndirs, nEC, nISO;
+    int64_t ec_base, iso_base, nE, nISOv;
+    const double *z;
+    int lut_exp, vec_ok;
+    double *scratch, *xout;
+    double *part, *epart;
+    unsigned *arrive;
+    f2 zero;                                  // 0 (dd2_fma_any)
+};
+
+}  // namespace detail
+}  // namespace cgb

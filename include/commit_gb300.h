@@ -121,6 +121,8 @@ int cgb_op_lut_grad(cgb_op *op, const double *x, const double *g, double *g_ic, 
  * Voxel shape of the float-float pair kernels: 1 the default (fewest padded samples), 2 a
  * warp per voxel, 0 = timed on the next call (the default at creation); set < 0 only reads.
  * *fwd / *adj (may be NULL) receive the shapes of A and A'.  Results agree to ~1e-16.
+ * Setting a shape also keeps this handle on the pair kernels (large products otherwise run
+ * with the LUT in shared memory).
  */
 int cgb_op_ff_shape(cgb_op *op, int set, int *fwd, int *adj);
 
@@ -344,6 +346,8 @@ int cgb_op_apply_batch(cgb_op *op, int adjoint, int nvec, const void *const *in,
  * set >= 0 stores a choice (0 = tune again on the next call, 1 or 2 = fixed), set < 0 only
  * reads; choice / ms_a / ms_b (may be NULL) receive the choice and the two measured times.
  * Both builds compute the same operations in the same order: results are identical.
+ * The float-float slots are those of the pair kernels: setting any choice also keeps this
+ * handle on them (large products otherwise run with the LUT in shared memory).
  */
 int cgb_op_occupancy(cgb_op *op, int slot, int set, int *choice, float *ms_a, float *ms_b);
 
