@@ -18,7 +18,7 @@
 #include <vector>
 
 #include "cgb_internal.cuh"
-#include "operator_pair.cuh"
+#include "fibre_sum.cuh"
 
 namespace cgb {
 
@@ -253,7 +253,7 @@ static int build_slabs(cgb_op *op, int want = 0) {
     CGB_CUDA(cudaMemcpy(dpos, pos.data(), pos.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     cudaError_t e = cudaMalloc((void **)&op->fib_slab, (size_t)(S + 1) * op->nF * sizeof(uint32_t));
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&op->fib_acc, (size_t)op->nF * (op->nIC > 0 ? op->nIC : 1) * sizeof(double));
+        e = cudaMalloc((void **)&op->fib_acc, (size_t)op->nF * (op->nIC > 0 ? op->nIC : 1) * fibre_lanes(op) * sizeof(double));
     op->fib_acc_slots = e == cudaSuccess ? 1 : 0;
     if (e != cudaSuccess) {
         cudaFree(dpos);
@@ -283,7 +283,7 @@ int cgb::ensure_fib_acc(cgb_op *op, int slots) {
     if (op->fib_acc) cudaFree(op->fib_acc);
     op->fib_acc = nullptr;
     op->fib_acc_slots = 0;
-    CGB_CUDA(cudaMalloc((void **)&op->fib_acc, (size_t)slots * op->nF * (op->nIC > 0 ? op->nIC : 1) * sizeof(double)));
+    CGB_CUDA(cudaMalloc((void **)&op->fib_acc, (size_t)slots * op->nF * (op->nIC > 0 ? op->nIC : 1) * fibre_lanes(op) * sizeof(double)));
     op->fib_acc_slots = slots;
     return CGB_OK;
 }

@@ -5,7 +5,7 @@
 #include <type_traits>
 
 #include "cgb_internal.cuh"
-#include "operator_pair.cuh"
+#include "fibre_sum.cuh"
 
 namespace cgb {
 
@@ -70,18 +70,6 @@ __global__ void k_f32_to_f64(const float *in, double *out, int64_t n) {
         out[i] = (double)in[i];
 }
 
-__global__ void k_fibre_sum32(const OpDev P, const float *__restrict__ scr, double *__restrict__ xout) {
-    const int64_t total = (int64_t)P.nF * P.nIC;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q / P.nF);
-        const uint32_t f = P.fib_order[q - (int64_t)i * P.nF];
-        const double s = fibre_gather_sum(P.fib_perm, scr + (size_t)i * P.n, P.fib_ptr[f], P.fib_ptr[f + 1], 0.0);
-        const int64_t c = (int64_t)i * P.nF + f;
-        xout[c] = s * (double)P.eval[c];
-    }
-}
-
 int grid_n(size_t n) {
     size_t g = (n + 255) / 256;
     if (g > 4096) g = 4096;
@@ -89,60 +77,16 @@ int grid_n(size_t n) {
     return (int)g;
 }
 
-int fibre_sum32(cgb_op *op, double *xout, cudaStream_t st) {
-    if (op->nIC > 0 && op->nF > 0) {
-        const int64_t total = (int64_t)op->nF * op->nIC;
-        int gb = (int)((total + 255) / 256);
-        if (gb > op->nsm * 16) gb = op->nsm * 16;
-        k_fibre_sum32<<<gb, 256, 0, st>>>(op->dev(), op->scratch32, xout);
-        CGB_CUDA(cudaGetLastError());
-    }
-    return CGB_OK;
-}
-
 }  // namespace
 
-__global__ void k_fibre_sum32_slab(const OpDev P, const float *__restrict__ scr, double *__restrict__ xout,
-                                   const uint32_t *__restrict__ fib_slab, double *__restrict__ accb, int s, int S) {
-    const int64_t total = (int64_t)P.nF * P.nIC;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q / P.nF);
-        const int64_t fq = q - (int64_t)i * P.nF;
-        const uint32_t beg = fib_slab[(size_t)s * P.nF + fq], end = fib_slab[(size_t)(s + 1) * P.nF + fq];
-        if (s > 0 && s < S - 1 && beg == end) continue;
-        const double acc = fibre_gather_sum(P.fib_perm, scr + (size_t)i * P.n, beg, end, s == 0 ? 0.0 : accb[q]);
-        if (s == S - 1) {
-            const int64_t c = (int64_t)i * P.nF + P.fib_order[fq];
-            xout[c] = acc * (double)P.eval[c];
-        } else {
-            accb[q] = acc;
-        }
-    }
-}
-
 int fibre_sum32_slab(cgb_op *op, const float *scr, double *xout, int s, cudaStream_t st, int slot) {
-    if (op->nIC > 0 && op->nF > 0) {
-        const int64_t total = (int64_t)op->nF * op->nIC;
-        if (slot >= op->fib_acc_slots) return fail(CGB_ERR_INVALID, "fibre pass: no accumulator for this vector");
-        int gb = (int)((total + 255) / 256);
-        if (gb > op->nsm * 16) gb = op->nsm * 16;
-        k_fibre_sum32_slab<<<gb, 256, 0, st>>>(op->dev(), scr, xout, op->fib_slab, op->fib_acc + (size_t)slot * total,
-                                                s, op->nslab);
-        CGB_CUDA(cudaGetLastError());
-    }
-    return CGB_OK;
+    if (slot >= op->fib_acc_slots) return fail(CGB_ERR_INVALID, "fibre pass: no accumulator for this vector");
+    double *acc = op->fib_acc + (size_t)slot * op->nF * op->nIC * fibre_lanes(op);
+    return launch_fibre_pass(op, scr, xout, acc, s, op->nslab, st);
 }
 
 int fibre_sum32_from(cgb_op *op, const float *scr, double *xout, cudaStream_t st) {
-    if (op->nIC > 0 && op->nF > 0) {
-        const int64_t total = (int64_t)op->nF * op->nIC;
-        int gb = (int)((total + 255) / 256);
-        if (gb > op->nsm * 16) gb = op->nsm * 16;
-        k_fibre_sum32<<<gb, 256, 0, st>>>(op->dev(), scr, xout);
-        CGB_CUDA(cudaGetLastError());
-    }
-    return CGB_OK;
+    return launch_fibre_pass(op, scr, xout, nullptr, 0, 1, st);
 }
 
 int forward_R2(cgb_op *, const RhsPtrs &, const float *, const float *, double *, cudaStream_t, int *);
@@ -271,7 +215,7 @@ static int adj_mix_slabs(cgb_op *op, int arith, const float *yin, int mode, cons
                          double *partials, cudaStream_t st, int *grid) {
     if (op->nslab <= 1) {
         CGB_TRY(adj_mix(op, arith, yin, mode, x, yobs, sqw, ax_a, ax_b, ca, cb, xout, partials, st, grid));
-        return fibre_sum32(op, xout, st);
+        return fibre_sum32_from(op, op->scratch32, xout, st);
     }
     int g = 0;
     CGB_TRY(slab_schedule(

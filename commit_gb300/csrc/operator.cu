@@ -1,6 +1,6 @@
 // Launch layer of the FP64-accurate operator: chooses the arithmetic policy, runs the
 // LUT-free kernels (setup_operator.py:713-915) and the per-fibre second pass of A'.
-#include "operator_kernels.cuh"
+#include "fibre_sum.cuh"
 
 #include <math.h>
 #include <string.h>
@@ -24,21 +24,6 @@ int adjoint_ff(cgb_op *op, const double *yin, int in_mode, const double *x, cons
                double *partials, cudaStream_t st, int *grid);
 
 namespace detail {
-// second A' pass: per-fibre sums of the voxel-ordered segment terms, fibres in the order
-// of their first segment (fib_order)
-__global__ void k_fibre_sum(const OpDev P, const double *__restrict__ scratch, double *__restrict__ xout) {
-    const int64_t total = (int64_t)P.nF * P.nIC;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q / P.nF);
-        const uint32_t f = P.fib_order[q - (int64_t)i * P.nF];
-        const uint32_t beg = P.fib_ptr[f], end = P.fib_ptr[f + 1];
-        const double s = fibre_gather_sum(P.fib_perm, scratch + (size_t)i * P.n, beg, end, 0.0);
-        const int64_t c = (int64_t)i * P.nF + f;
-        xout[c] = s * (double)P.eval[c];
-    }
-}
-
 // ------------------------------------------------------------------ LUT-free operator (nS == 1)
 __global__ void k_forward_nolut(const OpDev P, const double *__restrict__ x, double *__restrict__ yout,
                                 double *__restrict__ axout, const double *__restrict__ yobs,
@@ -106,28 +91,6 @@ __global__ void k_adjoint_nolut(const OpDev P, const double *__restrict__ yin, i
             for (uint32_t j = P.iso_ptr[v]; j < P.iso_ptr[v + 1]; ++j) xout[P.iso_base + P.iso_col[j]] = z;
     }
     if (partials) block_sum_store(nrm, partials + (size_t)blockIdx.x * kRedSlots);
-}
-
-// fibre pass of slab s, fibres in pass order (fib_order): the running sums continue from
-// acc (slab 0 starts at 0), terms in the fibre's position order, so the sums are those of
-// k_fibre_sum; the last slab applies eval and writes the fibre's column
-__global__ void k_fibre_sum_slab(const OpDev P, const double *__restrict__ scratch, double *__restrict__ xout,
-                                 const uint32_t *__restrict__ fib_slab, double *__restrict__ accb, int s, int S) {
-    const int64_t total = (int64_t)P.nF * P.nIC;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q / P.nF);
-        const int64_t fq = q - (int64_t)i * P.nF;
-        const uint32_t beg = fib_slab[(size_t)s * P.nF + fq], end = fib_slab[(size_t)(s + 1) * P.nF + fq];
-        if (s > 0 && s < S - 1 && beg == end) continue;
-        const double acc = fibre_gather_sum(P.fib_perm, scratch + (size_t)i * P.n, beg, end, s == 0 ? 0.0 : accb[q]);
-        if (s == S - 1) {
-            const int64_t c = (int64_t)i * P.nF + P.fib_order[fq];
-            xout[c] = acc * (double)P.eval[c];
-        } else {
-            accb[q] = acc;
-        }
-    }
 }
 
 // largest finite magnitude (as bits: non-negative floats order like their bit patterns)
@@ -203,27 +166,11 @@ int update_lut_exponents(cgb_op *op) {
 }
 
 int fibre_sum_slab(cgb_op *op, double *xout, int s, cudaStream_t st) {
-    if (op->nIC > 0 && op->nF > 0) {
-        const OpDev P = op->dev();
-        const int64_t total = (int64_t)op->nF * op->nIC;
-        int gb = (int)((total + 255) / 256);
-        if (gb > op->nsm * 16) gb = op->nsm * 16;
-        k_fibre_sum_slab<<<gb, 256, 0, st>>>(P, op->scratch, xout, op->fib_slab, op->fib_acc, s, op->nslab);
-        CGB_CUDA(cudaGetLastError());
-    }
-    return CGB_OK;
+    return launch_fibre_pass(op, op->scratch, xout, op->fib_acc, s, op->nslab, st);
 }
 
 int fibre_sum(cgb_op *op, double *xout, cudaStream_t st) {
-    if (op->nIC > 0 && op->nF > 0) {
-        const OpDev P = op->dev();
-        const int64_t total = (int64_t)op->nF * op->nIC;
-        int gb = (int)((total + 255) / 256);
-        if (gb > op->nsm * 16) gb = op->nsm * 16;
-        k_fibre_sum<<<gb, 256, 0, st>>>(P, op->scratch, xout);
-        CGB_CUDA(cudaGetLastError());
-    }
-    return CGB_OK;
+    return launch_fibre_pass(op, op->scratch, xout, nullptr, 0, 1, st);
 }
 
 static int run_forward(cgb_op *op, const double *x, double *y, double *ax, const double *yobs, const double *sqw,

@@ -83,7 +83,9 @@ __device__ __forceinline__ double widen_bits(float f) {
 
 __device__ __forceinline__ double widen(float f) {
     const unsigned a = __float_as_uint(f) & 0x7fffffffu;
-    return a - 0x00800000u < 0x7f000000u ? widen_bits(f) : (double)f;
+    double r = widen_bits(f);
+    if (a - 0x00800000u >= 0x7f000000u) r = a == 0u ? 0.0 : (double)f;
+    return r;
 }
 
 // s + e as a double (|e| is some units of the last place of s): one FP64 addition instead of
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_adjoint_p(const OpDev P, const
                             float s0, s1, e0, e1;
                             f2_unpack(tot.s, s0, s1);
                             f2_unpack(tot.e, e0, e1);
-                            double t = __shfl_sync(G.mask, ((double)s0 + (double)s1) + ((double)e0 + (double)e1), from, LPV);
+                            double t = __shfl_sync(G.mask, (widen(s0) + widen(s1)) + (widen(e0) + widen(e1)), from, LPV);
                             if (ez) t = t * pow2(ez);
                             if (mine) xout[cm.xbase + (size_t)i * cm.xstride + col] = t;
                         }

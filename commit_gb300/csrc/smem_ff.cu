@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
                 float s0, s1, e0, e1;
                 f2_unpack(P.s, s0, s1);
                 f2_unpack(P.e, e0, e1);
-                double t = ((double)s0 + (double)s1) + ((double)e0 + (double)e1);
+                double t = (widen(s0) + widen(s1)) + (widen(e0) + widen(e1));
                 t += __shfl_xor_sync(full, t, 1, 8);
                 if (sub == u) mine = t;
             }

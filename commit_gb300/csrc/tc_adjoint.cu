@@ -22,6 +22,7 @@
 // (tc_ptx.cuh).
 #include <cub/cub.cuh>
 
+#include "fibre_sum.cuh"
 #include "operator_launch.cuh"
 #include "tc_ptx.cuh"
 
@@ -462,25 +463,22 @@ __global__ void __launch_bounds__(kAThreads, 1) k_adjoint_tc(const TcAdjArgs A) 
 }
 
 // x[c] = eval[c] * sum of IC column c's terms (stored contiguously, in entry order, at
-// [fptr[c], fptr[c + 1])), FP64 sums; the columns in the order of their first entry (ford)
-__global__ void k_fibre_sum_entries(const uint32_t *__restrict__ fptr, const uint32_t *__restrict__ ford,
-                                    const float *__restrict__ terms, const uint32_t *__restrict__ eval, int64_t ncols,
-                                    double *__restrict__ xout) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < ncols;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = ford[q];
-        const uint32_t e = fptr[c + 1];
-        uint32_t k = fptr[c];
-        double s = 0.0;
-        for (; k + 8 <= e; k += 8) {
-            float t[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) t[u] = __ldg(terms + k + u);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) s += (double)t[u];
-        }
-        for (; k < e; ++k) s += (double)__ldg(terms + k);
-        xout[c] = s * (double)eval[c];
+// [fptr[c], fptr[c + 1])), FP64 sums by G lanes as in fibre_sum.cuh; the columns in the order
+// of their first entry (ford)
+template <int G>
+__global__ void __launch_bounds__(256) k_fibre_sum_entries(const uint32_t *__restrict__ fptr,
+                                                           const uint32_t *__restrict__ ford,
+                                                           const float *__restrict__ terms,
+                                                           const uint32_t *__restrict__ eval, int64_t ncols,
+                                                           double *__restrict__ xout) {
+    const int sub = threadIdx.x & (G - 1);
+    const int64_t step = (int64_t)gridDim.x * (256 / G);
+    for (int64_t q0 = blockIdx.x * (256ll / G) + (threadIdx.x & ~31) / G; q0 < ncols; q0 += step) {
+        const int64_t q = q0 + (threadIdx.x & 31) / G;
+        const uint32_t c = q < ncols ? ford[q] : 0u;
+        const uint32_t b = q < ncols ? fptr[c] : 0u, e = q < ncols ? fptr[c + 1] : 0u;
+        const double s = fibre_reduce<G>(fibre_lane_sum<G, float>(nullptr, terms, b, e, sub, 0.0));
+        if (q < ncols && sub == 0) xout[c] = s * (double)eval[c];
     }
 }
 
@@ -547,9 +545,11 @@ int adjoint_tc(cgb_op *op, int mode, const float *yin, const float *axa, const f
     CGB_CUDA(cudaGetLastError());
     const int64_t nic = (int64_t)op->nF * op->nIC;
     if (nic > 0) {
-        int64_t gb = (nic + 255) / 256;
-        if (gb > (int64_t)op->nsm * 16) gb = (int64_t)op->nsm * 16;
-        k_fibre_sum_entries<<<(int)gb, 256, 0, st>>>(op->tc_fptr, op->tc_ford, op->tc_terms, op->eval, nic, xout);
+        const int G = fibre_lanes(op);
+        int64_t gb = (nic * G + 255) / 256;
+        if (gb > (int64_t)op->nsm * 64) gb = (int64_t)op->nsm * 64;
+        auto kern = G == 1 ? k_fibre_sum_entries<1> : k_fibre_sum_entries<kFibreLanes>;
+        kern<<<(int)gb, 256, 0, st>>>(op->tc_fptr, op->tc_ford, op->tc_terms, op->eval, nic, xout);
         CGB_CUDA(cudaGetLastError());
     }
     if (grid) *grid = g;
