@@ -168,6 +168,7 @@ struct cgb_op {
     float *tc_terms;                // adjoint IC terms in entry order
     float *tc_ax;                   // A x rows for the gradient (FISTA), on demand
     __nv_bfloat16 *tc_rows16;       // EC rows (nEC * ndirs) then ISO rows (nISO) as BF16, stride tc_np
+    int lut_signed;                 // an IC table value is negative or not finite
     cgb::FfPlan *ffp;               // run layout of the shared-memory products, built on first use
     int ff_pinned;                  // a build or shape of the pair kernels was set: they run
     size_t bytes;
@@ -303,7 +304,8 @@ struct XScale {
     explicit XScale(cgb_op *o, bool on = true) : op(o) { op->xmax_on = on ? 1 : 0; }
     ~XScale() { op->xmax_on = 0; }
 };
-// exponents of the LUT bounds used by the range guard, from the device LUTs and lengths
+// exponents of the LUT bounds used by the range guard, from the device LUTs and lengths, and
+// whether the IC table has a negative or non-finite value
 int update_lut_exponents(cgb_op *op);
 
 // ------------------------------------------------------------------ occupancy autotuning

@@ -497,7 +497,7 @@ static int create_impl(int device, int nS, int ndirs, int nF, int64_t n, int nE,
     CGB_TRY(dalloc(op, &op->scratch, (size_t)n * (nIC > 0 ? nIC : 1)));
     CGB_TRY(dalloc(op, &op->partials, (size_t)partial_blocks(op) * kRedSlots));
     CGB_TRY(dalloc(op, &op->dscal, 64));
-    CGB_TRY(dalloc(op, &op->d_xmax, 1));
+    CGB_TRY(dalloc(op, &op->d_xmax, 2));
     CGB_CUDA(cudaMallocHost((void **)&op->h_scal, 64 * sizeof(double)));
     if (!nolut) CGB_TRY(update_lut_exponents(op));
     CGB_CUDA(cudaDeviceSynchronize());
@@ -578,8 +578,8 @@ int cgb_op_set_lut(cgb_op *op, const float *lutIC, const float *lutEC, const flo
                               cudaMemcpyDefault));
     }
     op->lut_r_kind = 0;  // reduced-precision copies are rebuilt on their next use
-    CGB_TRY(refresh_ff_plan(op));
-    return update_lut_exponents(op);
+    CGB_TRY(update_lut_exponents(op));
+    return refresh_ff_plan(op);
 }
 
 int cgb_op_ff_shape(cgb_op *op, int set, int *fwd, int *adj) {

@@ -122,6 +122,14 @@ __global__ void k_absmax_f32(const float *__restrict__ a, int64_t n, unsigned *_
     if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
+// set when a value is negative or not finite
+__global__ void k_signed_f32(const float *__restrict__ a, int64_t n, unsigned *__restrict__ out) {
+    bool bad = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bad |= !(a[i] >= 0.f && a[i] <= 3.0e38f);
+    if (bad) atomicOr(out, 1u);
+}
+
 }  // namespace detail
 
 using namespace detail;
@@ -137,9 +145,10 @@ int measure_input(cgb_op *op, const double *x, int64_t n, cudaStream_t st) {
 }
 
 int update_lut_exponents(cgb_op *op) {
-    // [0] max |LUT| over IC, EC and ISO, [1] max |IC length| (bits of non-negative floats)
+    // [0] max |LUT| over IC, EC and ISO, [1] max |IC length| (bits of non-negative floats),
+    // [2] whether an IC table value is negative or not finite
     unsigned *m = reinterpret_cast<unsigned *>(op->d_xmax);
-    CGB_CUDA(cudaMemset(m, 0, 2 * sizeof(unsigned)));
+    CGB_CUDA(cudaMemset(m, 0, 3 * sizeof(unsigned)));
     const struct {
         const float *p;
         int64_t n;
@@ -155,8 +164,16 @@ int update_lut_exponents(cgb_op *op) {
         k_absmax_f32<<<g, 256>>>(q.p, q.n, m + q.slot);
         CGB_CUDA(cudaGetLastError());
     }
-    unsigned h[2] = {0, 0};
+    const int64_t cells = (int64_t)op->nIC * op->ndirs * op->nS;
+    if (cells > 0) {
+        int g = (int)((cells + 255) / 256);
+        if (g > op->nsm * 8) g = op->nsm * 8;
+        k_signed_f32<<<g, 256>>>(op->lutIC, cells, m + 2);
+        CGB_CUDA(cudaGetLastError());
+    }
+    unsigned h[3] = {0, 0, 0};
     CGB_CUDA(cudaMemcpy(h, m, sizeof(h), cudaMemcpyDeviceToHost));
+    op->lut_signed = (int)h[2];
     float lut, len;
     memcpy(&lut, &h[0], 4);
     memcpy(&len, &h[1], 4);

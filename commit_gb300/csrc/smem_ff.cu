@@ -107,19 +107,11 @@ __global__ void k_col_max(const float *__restrict__ lut, int rows, int nS, int p
     colmax[s] = m;
 }
 
-// bit 0: a table entry is negative or not finite
-__global__ void k_table_flags(const float *__restrict__ lut, int64_t n, unsigned *__restrict__ flags) {
-    bool bad = false;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        bad |= !(lut[i] >= 0.f && lut[i] <= 3.0e38f);
-    if (bad) atomicOr(flags, 1u);
-}
-
 __global__ void k_eval_flags(const uint32_t *__restrict__ eval, int64_t n, unsigned *__restrict__ flags) {
     bool bad = false;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         bad |= eval[i] != 1u;
-    if (bad) atomicOr(flags, 2u);
+    if (bad) atomicOr(flags, 1u);
 }
 
 int grid_n(int64_t n) {
@@ -861,7 +853,7 @@ int build_plan(cgb_op *op, FfPlan *f) {
     const int64_t n = op->n;
     const int nV = op->nV;
     const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f), as = adj_shape(op->nIC, op->ndirs, op->nS, f);
-    if (!fs && !as) return CGB_OK;
+    if ((!fs && !as) || op->lut_signed) return CGB_OK;  // a negative or non-finite table entry: the pair kernels
     Buf bh, bi, bt, bk, bk2, bv, bf;
     uint32_t *head, *id;
     CGB_TRY(bh.get(&head, (size_t)n));
@@ -882,8 +874,6 @@ int build_plan(cgb_op *op, FfPlan *f) {
     CGB_TRY(bt.get(&tmp, b1 > b2 ? b1 : b2));
     CGB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, b1, head, id, (int)n));
     CGB_CUDA(cudaMemset(flags, 0, sizeof(unsigned)));
-    k_table_flags<<<grid_n((int64_t)op->nIC * op->ndirs * op->nS), 256>>>(
-        op->lutIC, (int64_t)op->nIC * op->ndirs * op->nS, flags);
     k_eval_flags<<<grid_n((int64_t)op->nF * op->nIC), 256>>>(op->eval, (int64_t)op->nF * op->nIC, flags);
     uint32_t lastid[2];
     unsigned hf = 0;
@@ -891,8 +881,7 @@ int build_plan(cgb_op *op, FfPlan *f) {
     CGB_CUDA(cudaMemcpy(&lastid[1], head + (n - 1), 4, cudaMemcpyDeviceToHost));
     CGB_CUDA(cudaMemcpy(&hf, flags, 4, cudaMemcpyDeviceToHost));
     f->nruns = (int64_t)lastid[0] + lastid[1];
-    f->eval_ones = !(hf & 2u);
-    if (hf & 1u) return CGB_OK;  // a negative or non-finite table entry: the pair kernels
+    f->eval_ones = hf == 0u;
     CGB_TRY(keep(op, &f->run_ptr, (size_t)nV + 1));
     CGB_TRY(keep(op, &f->run_o, (size_t)f->nruns));
     CGB_TRY(keep(op, &f->run_seg, (size_t)f->nruns + 1));
@@ -998,17 +987,8 @@ static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
 
 int refresh_ff_plan(cgb_op *op) {
     if (!op->ffp) return CGB_OK;
-    // new table: the sign check may change the choice of kernels, so the plan is laid out anew
-    // only when it does
-    Buf bf;
-    unsigned *flags, hf = 0;
-    CGB_TRY(bf.get(&flags, 1));
-    CGB_CUDA(cudaMemset(flags, 0, sizeof(unsigned)));
-    const int64_t cells = (int64_t)op->nIC * op->ndirs * op->nS;
-    k_table_flags<<<grid_n(cells), 256>>>(op->lutIC, cells, flags);
-    CGB_CUDA(cudaMemcpy(&hf, flags, 4, cudaMemcpyDeviceToHost));
     FfPlan *f = op->ffp;
-    if ((hf & 1u) || !f->run_ptr) {
+    if (op->lut_signed || !f->run_ptr) {  // the choice of kernels changed: laid out anew
         free_ff_plan(op);
         return CGB_OK;
     }
