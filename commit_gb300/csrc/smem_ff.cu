@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd_smem(const __grid_consta
     constexpr int NE = (NP + 1) & ~1, CS = 16 * NE, W = 16 * NP, GPB = kFwdThreads / 8;
     extern __shared__ __align__(16) float tab[];
     const unsigned full = 0xffffffffu;
-    const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3, par = grp & 1;
+    const int sub = threadIdx.x & 7, par = (threadIdx.x >> 3) & 1;
     const int chunk = blockIdx.x % A.nc, cta = blockIdx.x / A.nc, ncta = (gridDim.x - chunk + A.nc - 1) / A.nc;
     const int rows = A.nIC * A.ndirs;
     fill_table<kFwdThreads>(tab, A.img + (size_t)chunk * rows * CS, rows * CS);
@@ -203,19 +203,22 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd_smem(const __grid_consta
     const int ex = A.xmax ? ff_exp_hi((unsigned)(*A.xmax >> 32), A.lut_exp) : 0;
     const bool even = (A.nS & 1) == 0 && A.vec_ok;
     double nrm = 0.0;
+    // a warp takes four voxels at a time, neighbouring warps' fours going to different blocks (the
+    // voxels are sorted by run count: every block gets long and short ones)
     const int last = A.p1 - A.p0, stride = ncta * GPB;
+    const int lg = (int)((threadIdx.x & 31) >> 3), first = ((int)(threadIdx.x >> 5) * ncta + cta) * 4;
     // the voxel of the next step and its runs are fetched during this one
     auto voxel = [&](int pos) {
         int v = -1;
         if (pos < last) v = (int)A.vperm[A.p0 + pos];
         return v < A.v0 || v >= A.v1 ? -1 : v;
     };
-    int v = voxel(cta * GPB + grp), vn = voxel(cta * GPB + grp + stride);
+    int v = voxel(first + lg), vn = voxel(first + lg + stride);
     uint32_t rb = v >= 0 ? A.run_ptr[v] : 0u, re = v >= 0 ? A.run_ptr[v + 1] : 0u;
     fill_wait();
-    for (int w = cta * GPB; w < last; w += stride) {
+    for (int w = first; w < last; w += stride) {
         const uint32_t rbn = vn >= 0 ? A.run_ptr[vn] : 0u, ren = vn >= 0 ? A.run_ptr[vn + 1] : 0u;
-        const int vnn = voxel(w + grp + 2 * stride);
+        const int vnn = voxel(w + lg + 2 * stride);
         const uint32_t eb = v >= 0 && A.nEC ? A.ec_ptr[v] : 0u, ee = v >= 0 && A.nEC ? A.ec_ptr[v + 1] : 0u;
         const uint32_t ib = v >= 0 && A.nISO ? A.iso_ptr[v] : 0u, ie = v >= 0 && A.nISO ? A.iso_ptr[v + 1] : 0u;
         // largest coefficient and whether all are finite and >= 0
@@ -483,7 +486,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
         return *reinterpret_cast<const f2 *>(((k ^ 1) < NP ? (k & 1 ? tb1 : tb0) : tb) + row + 16 * k);
     };
     const bool even = (A.nS & 1) == 0 && A.vec_ok;
-    const int last = A.p1 - A.p0, stride = (int)(gridDim.x / parts) * GPB;
+    const int last = A.p1 - A.p0, ncta = (int)(gridDim.x / parts), stride = ncta * GPB;
     // the voxel of the next step, its first runs and its row are fetched during this one
     auto voxel = [&](int pos) {
         int v = -1;
@@ -491,14 +494,16 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
         return v < A.v0 || v >= A.v1 ? -1 : v;
     };
     const uint32_t *rb_of = A.run_blk + (size_t)blk * A.nV, *re_of = rb_of + A.nV;
-    const int first = (int)(blockIdx.x / parts) * GPB + (int)(threadIdx.x >> 3);
-    int v = voxel(first), vn = voxel(first + stride);
+    // fours of voxels interleaved over the blocks as in A
+    const int lg = (int)((threadIdx.x & 31) >> 3);
+    const int first = ((int)(threadIdx.x >> 5) * ncta + (int)(blockIdx.x / parts)) * 4;
+    int v = voxel(first + lg), vn = voxel(first + lg + stride);
     uint32_t rb = v >= 0 ? rb_of[v] : 0u, re = v >= 0 ? re_of[v] : 0u;
     unsigned on = rb + sub < re ? A.run_o[rb + sub] : 0u;  // orientation of this lane's next run
     fill_wait();
-    for (int w = first - (int)((threadIdx.x & 31) >> 3); w < last; w += stride) {  // w: the warp's first position
+    for (int w = first; w < last; w += stride) {  // w: the warp's first position
         const uint32_t rbn = vn >= 0 ? rb_of[vn] : 0u, ren = vn >= 0 ? re_of[vn] : 0u;
-        const int vnn = voxel(w + (int)((threadIdx.x & 31) >> 3) + 2 * stride);
+        const int vnn = voxel(w + lg + 2 * stride);
         f2 zh[NP], zl[NP];
         unsigned zmax = 0, neg = 0;
         auto load = [&](int k, double &z0, double &z1) {
