@@ -314,8 +314,8 @@ def workload_config(spec, D, K, args):
 
 def launches_per_pair(A, reduced: bool, tc: bool = False) -> int:
     """Kernels of one A + A' pair.  FP64 path: the max-|x| pass of the range guard and the
-    forward (large dense operators: the run coefficients before it), then per adjoint slab a
-    voxel pass and a fibre pass.  Reduced precision: the
+    forward (large operators: the run coefficients before it), then per adjoint slab a voxel
+    pass (large operators: the join of its parts) and a fibre pass.  Reduced precision: the
     FP32 -> FP64 column conversion and the forward, the adjoint (slab passes, or the
     tensor-core voxel pass and its fibre pass) and the FP64 -> FP32 conversion; the
     tensor-core forward adds its x*eval pass."""
@@ -324,8 +324,8 @@ def launches_per_pair(A, reduced: bool, tc: bool = False) -> int:
         return 3 + 3
     if reduced:
         return 2 + 2 * ns + 1
-    runs = A.ICn * A.ICnRF * A.nSAMPLES >= 2e7 and A.ICn * A.ICnRF >= 12 * A.ICnVOX
-    return 2 + int(runs) + 2 * ns
+    smem = A.ICn * A.ICnRF * A.nSAMPLES >= 1e7 and A.ICn * A.ICnRF >= 4 * -(-A.nSAMPLES // 96) * A.ICnVOX
+    return 3 + 3 * ns if smem else 2 + 2 * ns
 
 
 def traffic_for(args, spec, dom: str):

@@ -446,40 +446,32 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd_smem(const __grid_consta
 // ------------------------------------------------------------------ A'
 // 8 lanes own a voxel and hold the block's chunk of its input row as float-float pairs (pairs
 // laid out as in A); a batch of 8 runs is taken four at a time (butterfly reduce-scatter as
-// batch_dots_p).  With one chunk each lane writes the terms l * <L, z> of one run's segments;
-// with several the runs' parts go to `part`, and the warp that finishes its four voxels last
-// of the chunks adds them and writes the terms.  EC / ISO elements of four voxels are taken
+// batch_dots_p).  The runs' parts go to `part`; k_adj_join adds them and writes the terms
+// l * <L, z> of their segments (also with one chunk: the segment loads would be waited for in
+// the voxel pass).  EC / ISO elements of four voxels are taken
 // by the blocks of one of the orientation ranges in turn.
 
-// first two levels of the butterfly on four float-float pairs: lane sub is left with item
-// sub / 2, summed over half of the lanes
-__device__ __forceinline__ void scatter4(DD2 (&P)[4], int sub) {
+// First two levels of a butterfly reduce-scatter over four items: P[q] of lane sub is item
+// q ^ (sub >> 1) (each lane takes the items in its own order, so what it keeps is always in
+// front and no value is selected by lane); item sub >> 1, summed over the lanes of one parity,
+// is left in P[0].
+__device__ __forceinline__ void scatter4(DD2 (&P)[4]) {
     const unsigned full = 0xffffffffu;
 #pragma unroll
-    for (int h = 2, m = 4; h >= 1; h /= 2, m /= 2) {
-        const bool up = (sub & m) != 0;
+    for (int h = 2, m = 4; h >= 1; h /= 2, m /= 2)
 #pragma unroll
-        for (int j = 0; j < h; ++j) {
-            DD2 send, keep;
-            send.s = up ? P[j].s : P[j + h].s;
-            send.e = up ? P[j].e : P[j + h].e;
-            keep.s = up ? P[j + h].s : P[j].s;
-            keep.e = up ? P[j + h].e : P[j].e;
-            dd2_add(keep, dd2_shfl_xor(full, send, m, 8));
-            P[j] = keep;
-        }
-    }
+        for (int j = 0; j < h; ++j) dd2_add(P[j], dd2_shfl_xor(full, P[j + h], m, 8));
 }
 
 template <int NP>
-__global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_constant__ SmAdjArgs A) {
-    constexpr int NE = (NP + 1) & ~1, CS = 16 * NE, W = 16 * NP, GPB = kAdjThreads / 8;
+__global__ void __launch_bounds__(adj_threads(NP), 1) k_adj_smem(const __grid_constant__ SmAdjArgs A) {
+    constexpr int NE = (NP + 1) & ~1, CS = 16 * NE, W = 16 * NP, GPB = adj_threads(NP) / 8;
     extern __shared__ __align__(16) float tab[];
     const unsigned full = 0xffffffffu;
     const int sub = threadIdx.x & 7, par = (threadIdx.x >> 3) & 1;
     const int parts = A.nc * A.nb, part = blockIdx.x % parts, chunk = part / A.nb, blk = part % A.nb;
     const int s_base = chunk * W;
-    fill_table<kAdjThreads>(tab, A.img + (size_t)part * A.nIC * A.no * CS, A.nIC * A.no * CS);
+    fill_table<adj_threads(NP)>(tab, A.img + (size_t)part * A.nIC * A.no * CS, A.nIC * A.no * CS);
     auto kk = [&](int k) { return (k ^ 1) < NP ? k ^ par : k; };
     const float *tb = tab + 2 * sub, *tb0 = tb + 16 * par, *tb1 = tb - 16 * par;
     auto pair = [&](unsigned row, int k) {
@@ -499,7 +491,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
     const int first = ((int)(threadIdx.x >> 5) * ncta + (int)(blockIdx.x / parts)) * 4;
     int v = voxel(first + lg), vn = voxel(first + lg + stride);
     uint32_t rb = v >= 0 ? rb_of[v] : 0u, re = v >= 0 ? re_of[v] : 0u;
-    unsigned on = rb + sub < re ? A.run_o[rb + sub] : 0u;  // orientation of this lane's next run
+    const uint32_t own = (uint32_t)((sub & 1) * 4 + (sub >> 1));  // this lane's run of a batch
+    unsigned on = rb + own < re ? A.run_o[rb + own] : 0u;         // its orientation, of the next batch
     fill_wait();
     for (int w = first; w < last; w += stride) {  // w: the warp's first position
         const uint32_t rbn = vn >= 0 ? rb_of[vn] : 0u, ren = vn >= 0 ? re_of[vn] : 0u;
@@ -576,73 +569,84 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
         int most = (int)(re - rb);
         most = max(most, __shfl_xor_sync(full, most, 8));
         most = max(most, __shfl_xor_sync(full, most, 16));
-        if (most == 0) on = rbn + sub < ren ? __ldg(A.run_o + rbn + sub) : 0u;
+        if (most == 0) on = rbn + own < ren ? __ldg(A.run_o + rbn + own) : 0u;
+        // Eight runs at a time, four by four: run t of the batch belongs to lane (t & 3) * 2 + (t >> 2),
+        // which is where the butterfly leaves its dot product.
 #pragma unroll 1
         for (int b = 0; b < most; b += 8) {
-            const uint32_t j = rb + b + sub;
+            const uint32_t j = rb + b + own;
             const bool valid = j < re;
             const unsigned o = valid ? on - (unsigned)(blk * A.no) : 0u;
-            const int cnt = min(most - b, 8);
-            const uint32_t jn = b + 8 < most ? j + 8 : rbn + sub;
+            const uint32_t jn = b + 8 < most ? j + 8 : rbn + own;
             on = jn < (b + 8 < most ? re : ren) ? __ldg(A.run_o + jn) : 0u;
 #pragma unroll 1
             for (int i = 0; i < A.nIC; ++i) {
                 const unsigned row = ((unsigned)(i * A.no) + o) * (unsigned)CS;
-                float ds = 0.f, de = 0.f;
+                // four dot products' partial sums, of one sign (the bias is a power of two not above
+                // the sums: the difference is exact) or of any
+                auto four_pos = [&](int u) {
+                    DD2 P[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const unsigned r = __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8);
+                        const f2 L0 = pair(r, 0);
+                        const f2 s = f2_fma(zh[0], L0, bias);
+                        P[q].e = f2_fma(zl[0], L0, f2_fma(zh[0], L0, f2_sub(bias, s)));
+                        P[q].s = s;
+#pragma unroll
+                        for (int k = 1; k < NP; ++k) dd2_fma_same(P[q], zh[k], zl[k], pair(r, k));
+                        P[q].s = f2_sub(P[q].s, bias);
+                    }
+                    scatter4(P);
+                    return P[0];
+                };
+                auto four_any = [&](int u) {
+                    DD2 P[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const unsigned r = __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8);
+                        const f2 L0 = pair(r, 0);
+                        const f2 s = f2_fma(zh[0], L0, A.zero);
+                        P[q].e = f2_fma(zl[0], L0, f2_fma(zh[0], L0, f2_neg(s)));
+                        P[q].s = s;
+#pragma unroll
+                        for (int k = 1; k < NP; ++k) dd2_fma_any(P[q], zh[k], zl[k], pair(r, k), A.zero);
+                    }
+                    scatter4(P);
+                    return P[0];
+                };
+                // the lanes of even parity finish the first four, those of odd parity the others
+                DD2 M, N;
+                dd2_zero(M);
 #pragma unroll 1
-                for (int u = 0; u < cnt; u += 4) {
-                    // this lane's run is item src of the four
-                    const int src = sub - u;
-                    const bool me = src >= 0 && src < 4;
-                    DD2 P[4], M;
-                    if (any_pos) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const unsigned r = __shfl_sync(full, row, u + q, 8);
-                            P[q].s = bias;
-                            P[q].e = 0ull;
-#pragma unroll
-                            for (int k = 0; k < NP; ++k)
-                                dd2_fma_same(P[q], zh[k], zl[k], pair(r, k));
-                            // the bias is a power of two not above s: the difference is exact
-                            P[q].s = f2_sub(P[q].s, bias);
-                        }
-                        scatter4(P, sub);
-                        M = P[0];
+                for (int u = 0; u < 2; ++u) {
+                    N = M;
+                    if (u && b + 4 >= most) {
+                        dd2_zero(M);
+                        break;
                     }
+                    if (any_pos) M = four_pos(u);
                     if (any_mix) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const unsigned r = __shfl_sync(full, row, u + q, 8);
-                            dd2_zero(P[q]);
-#pragma unroll
-                            for (int k = 0; k < NP; ++k)
-                                dd2_fma_any(P[q], zh[k], zl[k], pair(r, k), A.zero);
-                        }
-                        scatter4(P, sub);
-                        if (!pos) M = P[0];
-                    }
-                    dd2_add(M, dd2_shfl_xor(full, M, 1, 8));
-                    float ts, te, s1, e1;
-                    f2_unpack(M.s, ts, s1);
-                    f2_unpack(M.e, te, e1);
-                    ff_add(ts, te, s1, e1);
-                    const float rs = __shfl_sync(full, ts, me ? src * 2 : 0, 8);
-                    const float rl = __shfl_sync(full, te, me ? src * 2 : 0, 8);
-                    if (me) {
-                        ds = rs;
-                        de = rl;
+                        const DD2 Q = four_any(u);
+                        if (any_pos) M.s = pos ? M.s : Q.s, M.e = pos ? M.e : Q.e;
+                        else M = Q;
                     }
                 }
+                const bool odd = (sub & 1) != 0;
+                DD2 send, keep;
+                send.s = odd ? N.s : M.s;  // N the first four, M the others
+                send.e = odd ? N.e : M.e;
+                keep.s = odd ? M.s : N.s;
+                keep.e = odd ? M.e : N.e;
+                dd2_add(keep, dd2_shfl_xor(full, send, 1, 8));
                 if (valid) {
+                    float ds, de, s1, e1;
+                    f2_unpack(keep.s, ds, s1);
+                    f2_unpack(keep.e, de, e1);
+                    ff_add(ds, de, s1, e1);
                     double t = ff_join(ds, de);
                     if (ez) t = t * pow2(ez);
-                    if (A.nc > 1) {
-                        A.part[((size_t)i * A.nruns + j) * A.nc + chunk] = t;
-                    } else {
-                        for (uint32_t g = A.run_seg[j]; g < A.run_seg[j + 1]; ++g)
-                            A.scratch[(size_t)i * A.n + g] = widen(A.seg_l[g]) * t;
-                    }
+                    A.part[((size_t)i * A.nruns + j) * A.nc + chunk] = t;
                 }
                 __syncwarp();
             }
@@ -695,11 +699,12 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
                                 A.zero);
                 dd2_add(P, dd2_shfl_xor(full, P, 4, 8));
                 dd2_add(P, dd2_shfl_xor(full, P, 2, 8));
-                // the last sums round at the size of the result: in FP64 for these single dots
+                // the last sum rounds at the size of the result: in FP64 for these single dots
                 float s0, s1, e0, e1;
                 f2_unpack(P.s, s0, s1);
                 f2_unpack(P.e, e0, e1);
-                double t = (widen(s0) + widen(s1)) + (widen(e0) + widen(e1));
+                ff_add(s0, e0, s1, e1);
+                double t = ff_join(s0, e0);
                 t += __shfl_xor_sync(full, t, 1, 8);
                 if (sub == u) mine = t;
             }
@@ -709,58 +714,47 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_smem(const __grid_consta
                 else A.xout[A.ec_base + col] = mine;
             }
         }
-        if (A.nc > 1) {
-            // the last of the chunks to finish these four voxels adds the parts
-            __threadfence();
-            __syncwarp();
-            unsigned before = 0;
-            unsigned *cell = A.arrive + (size_t)tile * A.nb + blk;
-            if ((threadIdx.x & 31) == 0) before = atomicAdd(cell, 1u);
-            before = __shfl_sync(full, before, 0);
-            if (before + 1u == (unsigned)A.nc) {
-                if ((threadIdx.x & 31) == 0) *cell = 0u;
-                __threadfence();
-                constexpr int U = 4;  // runs in flight per lane
-                for (uint32_t j0 = rb + sub; j0 < re; j0 += 8 * U) {
-                    uint32_t sb[U], se[U];
-                    float l[U];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const uint32_t j = min(j0 + 8 * u, re - 1);
-                        sb[u] = __ldg(A.run_seg + j);
-                        se[u] = j0 + 8 * u < re ? __ldg(A.run_seg + j + 1) : sb[u];
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u) l[u] = __ldg(A.seg_l + sb[u]);
-                    for (int i = 0; i < A.nIC; ++i) {
-                        double t[U];
-#pragma unroll
-                        for (int u = 0; u < U; ++u)
-                            t[u] = __ldcg(A.part + ((size_t)i * A.nruns + min(j0 + 8 * u, re - 1)) * A.nc);
-                        for (int c = 1; c < A.nc; ++c) {
-#pragma unroll
-                            for (int u = 0; u < U; ++u)
-                                t[u] += __ldcg(A.part + ((size_t)i * A.nruns + min(j0 + 8 * u, re - 1)) * A.nc + c);
-                        }
-#pragma unroll
-                        for (int u = 0; u < U; ++u)
-                            for (uint32_t g = sb[u]; g < se[u]; ++g)
-                                A.scratch[(size_t)i * A.n + g] = widen(g == sb[u] ? l[u] : __ldg(A.seg_l + g)) * t[u];
-                    }
-                }
-                for (int q0 = sub; q0 < tt; q0 += 8) {
-                    const int64_t col = column(q0);
-                    double t = __ldcg(A.epart + col * A.nc);
-                    for (int c = 1; c < A.nc; ++c) t += __ldcg(A.epart + col * A.nc + c);
-                    A.xout[A.ec_base + col] = t;
-                }
-            }
-            __syncwarp();
-        }
+        __syncwarp();
         v = vn;
         vn = vnn;
         rb = rbn;
         re = ren;
+    }
+}
+
+// Adds the chunks' parts for the voxels [v0, v1): terms l * <L, z> of the runs' segments, EC and
+// ISO columns.  A pass of its own streams the parts (1M streamlines: 2.4 GB, 0.7 ms); letting
+// the warp that finished a voxel last add them up cost 2.6 ms of latency in the voxel pass.
+__global__ void __launch_bounds__(256) k_adj_join(const SmAdjArgs A, const uint32_t *__restrict__ run_ptr) {
+    const int64_t first = blockIdx.x * 256ll + threadIdx.x, step = gridDim.x * 256ll;
+    const int64_t r0 = run_ptr[A.v0], r1 = run_ptr[A.v1];
+    for (int64_t r = r0 + first; r < r1; r += step) {
+        const uint32_t sb = A.run_seg[r], se = A.run_seg[r + 1];
+        const float l0 = A.seg_l[sb];
+        for (int i = 0; i < A.nIC; ++i) {
+            const double *q = A.part + ((size_t)i * A.nruns + r) * A.nc;
+            double t = q[0];
+            for (int c = 1; c < A.nc; ++c) t += q[c];
+            double *out = A.scratch + (size_t)i * A.n;
+            out[sb] = widen(l0) * t;
+            for (uint32_t g = sb + 1; g < se; ++g) out[g] = widen(A.seg_l[g]) * t;
+        }
+    }
+    auto column = [&](int64_t col) {
+        double t = A.epart[col * A.nc];
+        for (int c = 1; c < A.nc; ++c) t += A.epart[col * A.nc + c];
+        A.xout[A.ec_base + col] = t;
+    };
+    if (A.nc == 1) return;  // EC and ISO columns are written by the voxel pass
+    if (A.nEC) {
+        const int64_t e0 = A.ec_ptr[A.v0], e1 = A.ec_ptr[A.v1];
+        for (int64_t j = e0 + first; j < e1; j += step)
+            for (int i = 0; i < A.nEC; ++i) column((int64_t)i * A.nE + A.ec_col[j]);
+    }
+    if (A.nISO) {
+        const int64_t e0 = A.iso_ptr[A.v0], e1 = A.iso_ptr[A.v1];
+        for (int64_t j = e0 + first; j < e1; j += step)
+            for (int i = 0; i < A.nISO; ++i) column(A.iso_base - A.ec_base + (int64_t)i * A.nISOv + A.iso_col[j]);
     }
 }
 
@@ -903,13 +897,9 @@ int build_plan(cgb_op *op, FfPlan *f) {
     }
     if (as) {
         CGB_TRY(keep(op, &f->aimg, (size_t)f->anc * f->anb * op->nIC * f->ano * f->acs));
-        if (f->anc > 1) {
-            const size_t cells = 2 * ((size_t)nV / 4 + 1) * f->anb;
-            CGB_TRY(keep(op, &f->part, (size_t)op->nIC * f->nruns * f->anc));
+        CGB_TRY(keep(op, &f->part, (size_t)op->nIC * f->nruns * f->anc));
+        if (f->anc > 1)
             CGB_TRY(keep(op, &f->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * f->anc));
-            CGB_TRY(keep(op, &f->arrive, cells));
-            CGB_CUDA(cudaMemset(f->arrive, 0, cells * sizeof(unsigned)));
-        }
         CGB_TRY(keep(op, &f->run_blk, (size_t)(f->anb + 1) * nV));
         k_run_blk<<<(nV + 255) / 256, 256>>>(f->run_ptr, f->run_o, nV, f->anb, f->ano, f->run_blk);
     }
@@ -958,7 +948,7 @@ void free_ff_plan(cgb_op *op) {
     FfPlan *f = op->ffp;
     if (!f) return;
     void *p[] = {f->run_ptr, f->run_o, f->run_seg, f->coef, f->vperm, f->fimg, f->colmax, f->aimg, f->run_blk,
-                 f->part, f->epart, f->arrive, f->zrow};
+                 f->part, f->epart, f->zrow};
     for (void *q : p)
         if (q) cudaFree(q);
     if (f->done) cudaEventDestroy(f->done);
@@ -970,7 +960,7 @@ void free_ff_plan(cgb_op *op) {
 static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
     *out = nullptr;
     if (op->ff_variant != 1 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
-    if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork || !dense(op, kSmemMinItems)) return CGB_OK;
+    if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork) return CGB_OK;
     if (!op->ffp) {
         if (capturing(st)) return CGB_OK;
         static std::mutex m;
@@ -1006,7 +996,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     *ran = 0;
     FfPlan *f;
     CGB_TRY(plan_for(op, st, &f));
-    if (!f || !f->fwd_ok || !dense(op, kSmemMinItems)) return CGB_OK;
+    if (!f || !f->fwd_ok || !dense(op, smem_min_items(op->nS, f->fnc))) return CGB_OK;
     const OpDev P = op->dev();
     SmFwdArgs a;
     memset(&a, 0, sizeof(a));
@@ -1055,7 +1045,7 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
     *ran = 0;
     FfPlan *f;
     CGB_TRY(plan_for(op, st, &f));
-    if (!f || !f->adj_ok || !dense(op, 3 + 9 * f->anc)) return CGB_OK;
+    if (!f || !f->adj_ok || !dense(op, smem_min_items(op->nS, f->anc * f->anb))) return CGB_OK;
     const OpDev P = op->dev();
     SmAdjArgs a;
     memset(&a, 0, sizeof(a));
@@ -1069,21 +1059,23 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
     a.ec_base = P.ec_base; a.iso_base = P.iso_base; a.nE = op->nE; a.nISOv = op->nISOv;
     a.z = z; a.lut_exp = P.lut_exp_adj; a.vec_ok = (uintptr_t)z % 16 == 0;
     a.scratch = op->scratch; a.xout = xout; a.part = f->part; a.epart = f->epart;
-    // launches on the two streams of the slab schedule may overlap and share the four voxels
-    // at a boundary: they take the two halves of the arrival counts in turn
-    a.arrive = f->arrive + (f->flip ? ((size_t)op->nV / 4 + 1) * f->anb : 0);
-    f->flip ^= 1;
-    const int g = sm_grid(op, f->anc * f->anb, a.p1 - a.p0, kAdjThreads / 8);
+    const int g = sm_grid(op, f->anc * f->anb, a.p1 - a.p0, adj_threads(f->anp) / 8);
     const size_t smem = (size_t)op->nIC * f->ano * f->acs * sizeof(float);
     int rc = CGB_ERR_UNSUPPORTED;
     switch (f->anp) {
-        case 2: rc = launch_sm(k_adj_smem<2>, g, kAdjThreads, smem, st, a); break;
-        case 3: rc = launch_sm(k_adj_smem<3>, g, kAdjThreads, smem, st, a); break;
-        case 4: rc = launch_sm(k_adj_smem<4>, g, kAdjThreads, smem, st, a); break;
-        case 5: rc = launch_sm(k_adj_smem<5>, g, kAdjThreads, smem, st, a); break;
-        case 6: rc = launch_sm(k_adj_smem<6>, g, kAdjThreads, smem, st, a); break;
+        case 2: rc = launch_sm(k_adj_smem<2>, g, adj_threads(2), smem, st, a); break;
+        case 3: rc = launch_sm(k_adj_smem<3>, g, adj_threads(3), smem, st, a); break;
+        case 4: rc = launch_sm(k_adj_smem<4>, g, adj_threads(4), smem, st, a); break;
+        case 5: rc = launch_sm(k_adj_smem<5>, g, adj_threads(5), smem, st, a); break;
+        case 6: rc = launch_sm(k_adj_smem<6>, g, adj_threads(6), smem, st, a); break;
     }
     CGB_TRY(rc);
+    {
+        const int64_t runs = f->nruns * (a.v1 - a.v0) / op->nV + 1;
+        const int64_t blocks = (runs + 255) / 256, cap = (int64_t)op->nsm * 32;
+        k_adj_join<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(a, f->run_ptr);
+        CGB_CUDA(cudaGetLastError());
+    }
     *ran = 1;
     return CGB_OK;
 }
@@ -1096,7 +1088,7 @@ int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, 
     *z = nullptr;
     FfPlan *f;
     CGB_TRY(plan_for(op, st, &f));
-    if (!f || !f->adj_ok || !f->fwd_ok || !dense(op, 3 + 9 * f->anc)) return CGB_OK;
+    if (!f || !f->adj_ok || !f->fwd_ok || !dense(op, smem_min_items(op->nS, f->anc * f->anb))) return CGB_OK;
     if (!f->zrow) {
         if (capturing(st)) return CGB_OK;
         CGB_TRY(keep(op, &f->zrow, (size_t)op->nrows));

@@ -8,8 +8,8 @@
 //   A   the block holds a chunk of the samples for every orientation and computes these
 //       samples of every row (no partial results leave the block);
 //   A'  the block holds a chunk of the samples for a range of orientations (all of them when
-//       they fit) and computes these samples' part of the runs' dot products; the block that
-//       finishes a few voxels last adds their parts up, from L2.
+//       they fit) and computes these samples' part of the runs' dot products; a streaming pass
+//       adds the parts up.
 // The runs (segments of a voxel with one orientation) are laid out once per handle
 // (FfPlan); A first forms each run's coefficient sum(l * x * eval) in one pass.
 //
@@ -48,8 +48,6 @@ struct FfPlan {
     uint32_t *run_blk;           // [anb + 1][nV] first run of the voxel in a range
     double *part;                // [nIC * nruns][anc] parts of the runs' dot products (anc > 1)
     double *epart;               // [EC and ISO columns][anc]
-    unsigned *arrive;            // [2][voxels / 4 * anb] parts finished per four voxels
-    int flip;                    // half of arrive of the last launch (two may overlap)
     double *zrow;                // [nrows] weighted residual (FISTA gradient)
     cudaEvent_t done;            // the last product that used coef has finished
     cudaStream_t last;           // ... and its stream
@@ -57,17 +55,25 @@ struct FfPlan {
 };
 
 constexpr int kVoxWindow = 4096;
-constexpr int kFwdThreads = 768, kAdjThreads = 768;  // one block per SM, 80 registers a thread
+// threads of the one block per SM: 80 registers a thread, and 96 where A' needs them (measured at 5
+// and 6 pairs per lane: 45 and 1900 us with 640 threads, 49 and 1940 with 768; at 4: 616 and 571)
+constexpr int kFwdThreads = 768;
+constexpr int adj_threads(int np) { return np <= 4 ? 768 : 640; }
 // Where the shared-memory kernels take over from the pair kernels of operator_pair.cuh: a
 // product of at least kSmemMinWork terms (segments x responses x samples) with at least
-// kSmemMinItems (A) or 3 + 9 * chunks (A') segments x responses per voxel.  Measured, us, here /
-// pair kernels: A 38 / 29 at 8 M terms, 43 / 38 at 17 M, 50 / 58 at 26 M; 101 / 116 at 13 per
-// voxel, 351 / 318 at 10 and 56 / 52 at 5.  A' per voxel: one chunk 139 / 150 at 13 (66 samples),
-// two 337 / 299 at 8 and 270 / 367 at 27 (145 and 99 samples), three 3461 / 3354 at 20 and
-// 2155 / 2541 at 33 (288 samples).  Below the lines the table fill (160-190 KB per SM) and the
-// per-voxel steps, repeated for every chunk, cost more than the gathers from L2.
-constexpr double kSmemMinWork = 2e7;
-constexpr double kSmemMinItems = 12;
+// smem_min_items() segments x responses per voxel: 4 for every chunk the sample count asks for,
+// 8 for every further part that the table's size adds.  Measured, us, here / pair kernels:
+//   terms      A 36 / 28 and A' 35 / 32 at 8 M, 39 / 41 and 40 / 46 at 12 M, 45 / 58 and 46 / 65 at 26 M;
+//   per voxel  66 samples A 48 / 52, A' 48 / 59 at 5; 145 samples (2 chunks) 191 / 230, 209 / 275 at
+//              8; 288 samples (3 chunks) 1096 / 1241, 1030 / 1556 at 13 and 1575 / 2251, 1534 / 2515 at 33;
+//              2 responses x 66 samples (A 3 chunks for 1, A' 2 ranges) 345 / 319, 371 / 370 at 10.
+// Below the lines the table fill (160-190 KB per SM) and the per-voxel steps, repeated for
+// every part, cost more than the gathers from L2.
+constexpr double kSmemMinWork = 1e7;
+inline double smem_min_items(int nS, int parts) {
+    const int chunks = (nS + 95) / 96;
+    return 4.0 * chunks + 8.0 * (parts - chunks);
+}
 
 namespace detail {
 
@@ -159,7 +165,6 @@ struct SmAdjArgs {
     int lut_exp, vec_ok;
     double *scratch, *xout;
     double *part, *epart;
-    unsigned *arrive;
     f2 zero;                                  // 0 (dd2_fma_any)
 };
 
