@@ -168,7 +168,7 @@ struct cgb_op {
     float *tc_terms;                // adjoint IC terms in entry order
     float *tc_ax;                   // A x rows for the gradient (FISTA), on demand
     __nv_bfloat16 *tc_rows16;       // EC rows (nEC * ndirs) then ISO rows (nISO) as BF16, stride tc_np
-    int lut_signed;                 // an IC table value is negative or not finite
+    int lut_signed;                 // bit 0: an IC table value is negative or not finite, bit 1: any table value is not finite
     cgb::FfPlan *ffp;               // run layout of the shared-memory products, built on first use
     int ff_pinned;                  // a build or shape of the pair kernels was set: they run
     size_t bytes;

@@ -122,12 +122,14 @@ __global__ void k_absmax_f32(const float *__restrict__ a, int64_t n, unsigned *_
     if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
-// set when a value is negative or not finite
-__global__ void k_signed_f32(const float *__restrict__ a, int64_t n, unsigned *__restrict__ out) {
-    bool bad = false;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        bad |= !(a[i] >= 0.f && a[i] <= 3.0e38f);
-    if (bad) atomicOr(out, 1u);
+// bit 0: a value is negative or not finite; bit 1: a value is not finite
+__global__ void k_signed_f32(const float *__restrict__ a, int64_t n, unsigned bits, unsigned *__restrict__ out) {
+    unsigned m = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (!(a[i] >= 0.f)) m |= 1u;
+        if (!(fabsf(a[i]) <= 3.0e38f)) m |= 3u;
+    }
+    if (m & bits) atomicOr(out, m & bits);
 }
 
 }  // namespace detail
@@ -146,7 +148,7 @@ int measure_input(cgb_op *op, const double *x, int64_t n, cudaStream_t st) {
 
 int update_lut_exponents(cgb_op *op) {
     // [0] max |LUT| over IC, EC and ISO, [1] max |IC length| (bits of non-negative floats),
-    // [2] whether an IC table value is negative or not finite
+    // [2] bit 0: an IC table value is negative or not finite, bit 1: any table value is not finite
     unsigned *m = reinterpret_cast<unsigned *>(op->d_xmax);
     CGB_CUDA(cudaMemset(m, 0, 3 * sizeof(unsigned)));
     const struct {
@@ -162,13 +164,7 @@ int update_lut_exponents(cgb_op *op) {
         int g = (int)((q.n + 255) / 256);
         if (g > op->nsm * 8) g = op->nsm * 8;
         k_absmax_f32<<<g, 256>>>(q.p, q.n, m + q.slot);
-        CGB_CUDA(cudaGetLastError());
-    }
-    const int64_t cells = (int64_t)op->nIC * op->ndirs * op->nS;
-    if (cells > 0) {
-        int g = (int)((cells + 255) / 256);
-        if (g > op->nsm * 8) g = op->nsm * 8;
-        k_signed_f32<<<g, 256>>>(op->lutIC, cells, m + 2);
+        if (q.slot == 0) k_signed_f32<<<g, 256>>>(q.p, q.n, q.p == op->lutIC ? 3u : 2u, m + 2);
         CGB_CUDA(cudaGetLastError());
     }
     unsigned h[3] = {0, 0, 0};

@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd_smem(const __grid_consta
             for (int b = 0; b < m; b += 8) {
                 const int q = b + sub;
                 float h = 0.f, l = 0.f;
-                const float *row = A.lutISO;
+                const float *row = A.nISO ? A.lutISO : A.lutEC;  // lanes past the end read (and drop) a row that exists
                 if (q < tt) {
                     double xv;
                     if (q < te) {
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(adj_threads(NP), 1) k_adj_smem(const __grid_co
 #pragma unroll 1
         for (int b = 0; b < m; b += 8) {
             const int q0 = b + sub;
-            const float *row = A.lutISO;
+            const float *row = A.nISO ? A.lutISO : A.lutEC;
             int64_t col = -1;
             if (q0 < tt) {
                 col = column(q0);
@@ -852,7 +852,7 @@ int build_plan(cgb_op *op, FfPlan *f) {
     const int64_t n = op->n;
     const int nV = op->nV;
     const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f), as = adj_shape(op->nIC, op->ndirs, op->nS, f);
-    if ((!fs && !as) || op->lut_signed) return CGB_OK;  // a negative or non-finite table entry: the pair kernels
+    if ((!fs && !as) || op->lut_signed) return CGB_OK;  // the pair kernels skip zero coefficients, these may multiply by one
     Buf bh, bi, bt, bk, bk2, bv, bf;
     uint32_t *head, *id;
     CGB_TRY(bh.get(&head, (size_t)n));
@@ -944,15 +944,19 @@ int launch_sm(F kern, int grid, int threads, size_t smem, cudaStream_t st, const
 
 }  // namespace
 
-void free_ff_plan(cgb_op *op) {
-    FfPlan *f = op->ffp;
-    if (!f) return;
+static void drop_plan(FfPlan *f) {
     void *p[] = {f->run_ptr, f->run_o, f->run_seg, f->coef, f->vperm, f->fimg, f->colmax, f->aimg, f->run_blk,
                  f->part, f->epart, f->zrow};
     for (void *q : p)
         if (q) cudaFree(q);
     if (f->done) cudaEventDestroy(f->done);
-    delete f;
+    memset((void *)f, 0, sizeof(*f));
+}
+
+void free_ff_plan(cgb_op *op) {
+    if (!op->ffp) return;
+    drop_plan(op->ffp);
+    delete op->ffp;
     op->ffp = nullptr;
 }
 
@@ -968,12 +972,18 @@ static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
         if (!op->ffp) {
             FfPlan *f = new FfPlan();
             memset((void *)f, 0, sizeof(*f));
-            op->ffp = f;
+            const size_t bytes = op->bytes;
             const int rc = build_plan(op, f);
             if (rc != CGB_OK) {
-                free_ff_plan(op);
-                return rc;
+                drop_plan(f);
+                op->bytes = bytes;
+                if (rc != CGB_ERR_NOMEM) {
+                    delete f;
+                    return rc;
+                }
+                cudaGetLastError();  // no room for the plan: it stays empty and the pair kernels run
             }
+            op->ffp = f;
         }
     }
     *out = op->ffp;
@@ -1091,7 +1101,13 @@ int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, 
     if (!f || !f->adj_ok || !f->fwd_ok || !dense(op, smem_min_items(op->nS, f->anc * f->anb))) return CGB_OK;
     if (!f->zrow) {
         if (capturing(st)) return CGB_OK;
-        CGB_TRY(keep(op, &f->zrow, (size_t)op->nrows));
+        const int rc = keep(op, &f->zrow, (size_t)op->nrows);
+        if (rc == CGB_ERR_NOMEM) {
+            cudaGetLastError();
+            f->zrow = nullptr;
+            return CGB_OK;
+        }
+        CGB_TRY(rc);
     }
     if (in_mode == 1) {
         int ran = 0;

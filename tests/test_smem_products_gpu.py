@@ -143,6 +143,26 @@ def test_non_finite_input_stays_in_its_voxels(bad):
     assert np.array_equal(~np.isfinite(g), hit)
 
 
+@pytest.mark.parametrize('table', ['wmh', 'iso'])
+def test_non_finite_table_rows_stay_in_their_voxels(table):
+    """A zero coefficient skips its row also where a neighbour's does not: an Inf in an EC or ISO
+    row reaches only the voxels with a coefficient for it."""
+    from commit_gb300.operator import LinearOperator
+    D, K = _problem(97, 6000)
+    K = dict(K, **{table: K[table].copy()})
+    o = int(np.bincount(D['EC']['dir']).argmax())
+    K[table].reshape(-1, 97)[o if table == 'wmh' else 0, 3] = np.inf
+    A = LinearOperator(D, K, None)
+    x = np.random.default_rng(7).uniform(0.1, 1, A.nCOLS)
+    base, comp = (D['IC']['nSTR'], 'EC') if table == 'wmh' else (D['IC']['nSTR'] + D['EC']['n'], 'ISO')
+    n = D[comp]['n']
+    x[base:base + n:2] = 0.0
+    rows = D[comp]['dir'] == o if comp == 'EC' else np.ones(n, bool)
+    hit = np.unique(D[comp]['vox'][rows & (x[base:base + n] != 0)])
+    r = A.dot(torch.from_numpy(x).cuda()).cpu().numpy().reshape(-1, 97)
+    assert hit.size and np.array_equal(np.flatnonzero(~np.isfinite(r).all(1)), hit)
+
+
 def test_fit_matches_the_oracle():
     """FISTA on the residual rows of the shared-memory gradient, host loop and graph."""
     from commit_gb300 import solvers, synth
