@@ -153,12 +153,16 @@ int cgb_op_apply(cgb_op *op, int adjoint, const void *in, int64_t in_len, void *
         if (arith != CGB_ARITH_BF16 && arith != CGB_ARITH_FP16 && arith != CGB_ARITH_F32)
             return fail(CGB_ERR_INVALID, "FP32 vectors need arith BF16, FP16 or F32");
         if (!op->d_x64) CGB_CUDA(cudaMalloc((void **)&op->d_x64, (op->ncols > 0 ? op->ncols : 1) * sizeof(double)));
+        int ran = 0;
         if (!adjoint) {
+            CGB_TRY(forward_smem_mix(op, (const float *)in, (float *)out, st, arith, &ran));
+            if (ran) return CGB_OK;
             CGB_TRY(convert_f32_to_f64((const float *)in, op->d_x64, op->ncols, st));
             return launch_resnorm_mix(op, op->d_x64, nullptr, nullptr, nullptr, nullptr, (float *)out, st, arith,
                                       nullptr);
         }
-        CGB_TRY(launch_adjoint_mix(op, (const float *)in, op->d_x64, st, arith));
+        CGB_TRY(adjoint_smem_mix(op, (const float *)in, op->d_x64, st, arith, &ran));
+        if (!ran) CGB_TRY(launch_adjoint_mix(op, (const float *)in, op->d_x64, st, arith));
         return convert_f64_to_f32(op->d_x64, (float *)out, op->ncols, st);
     }
     return fail(CGB_ERR_UNSUPPORTED, "unsupported dtype / arithmetic combination");

@@ -92,7 +92,9 @@ struct RhsPtrs {
     int active[kMaxRhs];            // 0: skip this vector (outputs untouched)
 };
 
+struct RunLayout;                   // runs of segments (smem_ff.cuh)
 struct FfPlan;                      // shared-memory float-float products (smem_ff.cuh)
+struct MixPlan;                     // shared-memory reduced-precision products (smem_mix.cuh)
 
 }  // namespace cgb
 
@@ -169,6 +171,9 @@ struct cgb_op {
     float *tc_ax;                   // A x rows for the gradient (FISTA), on demand
     __nv_bfloat16 *tc_rows16;       // EC rows (nEC * ndirs) then ISO rows (nISO) as BF16, stride tc_np
     int lut_signed;                 // bit 0: an IC table value is negative or not finite, bit 1: any table value is not finite
+    cgb::RunLayout *runs;           // built on the first product that uses them
+    cgb::MixPlan *mixp;             // buffers of the FP32-vector products, likewise
+    int mixp_kind;                  // arithmetic of its table image (0: to be filled)
     cgb::FfPlan *ffp;               // run layout of the shared-memory products, built on first use
     int ff_pinned;                  // a build or shape of the pair kernels was set: they run
     size_t bytes;
@@ -201,6 +206,13 @@ int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, 
                   const double **z);
 int refresh_ff_plan(cgb_op *op);
 void free_ff_plan(cgb_op *op);
+int ensure_runs(cgb_op *op);
+void free_runs(cgb_op *op);
+// reduced-precision products of FP32 vectors with the table in shared memory (smem_mix_*.cu); `ran`
+// = 0: the other kernels are to do it
+int forward_smem_mix(cgb_op *op, const float *x, float *y, cudaStream_t st, int arith, int *ran);
+int adjoint_smem_mix(cgb_op *op, const float *y, double *x, cudaStream_t st, int arith, int *ran);
+void free_mix_plan(cgb_op *op);
 int reduction_blocks(const cgb_op *op);
 void free_grad_state(cgb_op *op);
 // reduced-precision path (mixed.cu): FP32 rows, FP64 columns

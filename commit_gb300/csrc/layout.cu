@@ -292,6 +292,8 @@ static void free_op(cgb_op *op) {
     if (!op) return;
     free_grad_state(op);
     free_ff_plan(op);
+    free_mix_plan(op);
+    free_runs(op);
     void *ptrs[] = {op->lutIC, op->lutEC, op->lutISO, op->lutIC_p, op->lutEC_p, op->lutISO_p, op->lutIC_r, op->lutEC_r, op->lutISO_r, op->seg_l16, op->vox_ptr,
                     op->seg_f, op->eval, op->fib_ptr, op->fib_perm, op->fib_order, op->ec_ptr, op->ec_col, op->iso_ptr,
                     op->iso_col, op->seg_o, op->ec_o, op->seg_l, op->scratch, op->scratch32, op->partials,
@@ -578,6 +580,7 @@ int cgb_op_set_lut(cgb_op *op, const float *lutIC, const float *lutEC, const flo
                               cudaMemcpyDefault));
     }
     op->lut_r_kind = 0;  // reduced-precision copies are rebuilt on their next use
+    op->mixp_kind = 0;
     CGB_TRY(update_lut_exponents(op));
     return refresh_ff_plan(op);
 }

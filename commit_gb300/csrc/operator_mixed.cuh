@@ -20,17 +20,21 @@ struct LutPair;
 
 template <>
 struct LutPair<__nv_bfloat16> {
-    __device__ static __forceinline__ f2 ld(const __nv_bfloat16 *p) {
-        const unsigned int u = __ldg(reinterpret_cast<const unsigned int *>(p));
-        // bf16 -> f32 is a 16-bit left shift of each half
+    // bf16 -> f32 is a 16-bit left shift of each half
+    __device__ static __forceinline__ f2 conv(unsigned u) {
         return f2_pack(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+    }
+    __device__ static __forceinline__ f2 ld(const __nv_bfloat16 *p) {
+        return conv(__ldg(reinterpret_cast<const unsigned int *>(p)));
     }
 };
 
 template <>
 struct LutPair<__half> {
     __device__ static __forceinline__ f2 ld(const __half *p) {
-        const unsigned int u = __ldg(reinterpret_cast<const unsigned int *>(p));
+        return conv(__ldg(reinterpret_cast<const unsigned int *>(p)));
+    }
+    __device__ static __forceinline__ f2 conv(unsigned u) {
         __half2 h;
         memcpy(&h, &u, 4);
         const float2 f = __half22float2(h);

@@ -834,6 +834,13 @@ bool adj_shape(int nIC, int ndirs, int nS, FfPlan *f) {
     return best <= 16;
 }
 
+void drop_runs(RunLayout *R) {
+    void *p[] = {R->run_ptr, R->run_o, R->run_seg, R->vperm};
+    for (void *q : p)
+        if (q) cudaFree(q);
+    delete R;
+}
+
 int build_images(cgb_op *op, FfPlan *f) {
     const int rows = op->nIC * op->ndirs;
     if (f->fimg)
@@ -848,11 +855,9 @@ int build_images(cgb_op *op, FfPlan *f) {
     return CGB_OK;
 }
 
-int build_plan(cgb_op *op, FfPlan *f) {
+int build_runs(cgb_op *op, RunLayout *R) {
     const int64_t n = op->n;
     const int nV = op->nV;
-    const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f), as = adj_shape(op->nIC, op->ndirs, op->nS, f);
-    if ((!fs && !as) || op->lut_signed) return CGB_OK;  // the pair kernels skip zero coefficients, these may multiply by one
     Buf bh, bi, bt, bk, bk2, bv, bf;
     uint32_t *head, *id;
     CGB_TRY(bh.get(&head, (size_t)n));
@@ -879,29 +884,39 @@ int build_plan(cgb_op *op, FfPlan *f) {
     CGB_CUDA(cudaMemcpy(&lastid[0], id + (n - 1), 4, cudaMemcpyDeviceToHost));
     CGB_CUDA(cudaMemcpy(&lastid[1], head + (n - 1), 4, cudaMemcpyDeviceToHost));
     CGB_CUDA(cudaMemcpy(&hf, flags, 4, cudaMemcpyDeviceToHost));
-    f->nruns = (int64_t)lastid[0] + lastid[1];
-    f->eval_ones = hf == 0u;
-    CGB_TRY(keep(op, &f->run_ptr, (size_t)nV + 1));
-    CGB_TRY(keep(op, &f->run_o, (size_t)f->nruns));
-    CGB_TRY(keep(op, &f->run_seg, (size_t)f->nruns + 1));
-    CGB_TRY(keep(op, &f->vperm, (size_t)nV));
+    R->nruns = (int64_t)lastid[0] + lastid[1];
+    R->eval_ones = hf == 0u;
+    CGB_TRY(keep(op, &R->run_ptr, (size_t)nV + 1));
+    CGB_TRY(keep(op, &R->run_o, (size_t)R->nruns));
+    CGB_TRY(keep(op, &R->run_seg, (size_t)R->nruns + 1));
+    CGB_TRY(keep(op, &R->vperm, (size_t)nV));
+    k_run_fill<<<grid_n(n), 256>>>(head, id, op->seg_o, n, (uint32_t)R->nruns, R->run_o, R->run_seg);
+    k_run_ptr<<<(nV + 256) / 256, 256>>>(op->vox_ptr, id, nV, n, (uint32_t)R->nruns, R->run_ptr);
+    k_perm_key<<<(nV + 255) / 256, 256>>>(R->run_ptr, nV, key, val);
+    CGB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, b2, key, key2, val, R->vperm, nV, 0, 64));
+    CGB_CUDA(cudaDeviceSynchronize());
+    return CGB_OK;
+}
+
+int build_plan(cgb_op *op, FfPlan *f) {
+    const int nV = op->nV;
+    const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f), as = adj_shape(op->nIC, op->ndirs, op->nS, f);
+    if ((!fs && !as) || op->lut_signed) return CGB_OK;  // the pair kernels skip zero coefficients, these may multiply by one
+    CGB_TRY(ensure_runs(op));
+    const RunLayout *R = op->runs;
     CGB_TRY(keep(op, &f->colmax, (size_t)kMaxSamples + 128));
-    k_run_fill<<<grid_n(n), 256>>>(head, id, op->seg_o, n, (uint32_t)f->nruns, f->run_o, f->run_seg);
-    k_run_ptr<<<(nV + 256) / 256, 256>>>(op->vox_ptr, id, nV, n, (uint32_t)f->nruns, f->run_ptr);
-    k_perm_key<<<(nV + 255) / 256, 256>>>(f->run_ptr, nV, key, val);
-    CGB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, b2, key, key2, val, f->vperm, nV, 0, 64));
     if (fs) {
         CGB_TRY(keep(op, &f->fimg, (size_t)f->fnc * op->nIC * op->ndirs * f->fcs));
-        CGB_TRY(keep(op, &f->coef, (size_t)op->nIC * f->nruns));
+        CGB_TRY(keep(op, &f->coef, (size_t)op->nIC * R->nruns));
         CGB_CUDA(cudaEventCreateWithFlags(&f->done, cudaEventDisableTiming));
     }
     if (as) {
         CGB_TRY(keep(op, &f->aimg, (size_t)f->anc * f->anb * op->nIC * f->ano * f->acs));
-        CGB_TRY(keep(op, &f->part, (size_t)op->nIC * f->nruns * f->anc));
+        CGB_TRY(keep(op, &f->part, (size_t)op->nIC * R->nruns * f->anc));
         if (f->anc > 1)
             CGB_TRY(keep(op, &f->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * f->anc));
         CGB_TRY(keep(op, &f->run_blk, (size_t)(f->anb + 1) * nV));
-        k_run_blk<<<(nV + 255) / 256, 256>>>(f->run_ptr, f->run_o, nV, f->anb, f->ano, f->run_blk);
+        k_run_blk<<<(nV + 255) / 256, 256>>>(R->run_ptr, R->run_o, nV, f->anb, f->ano, f->run_blk);
     }
     CGB_TRY(build_images(op, f));
     CGB_CUDA(cudaDeviceSynchronize());
@@ -944,9 +959,29 @@ int launch_sm(F kern, int grid, int threads, size_t smem, cudaStream_t st, const
 
 }  // namespace
 
+// the handle's runs, laid out on first use (not under stream capture: the callers see to it)
+int ensure_runs(cgb_op *op) {
+    static std::mutex m;
+    std::lock_guard<std::mutex> g(m);
+    if (op->runs) return CGB_OK;
+    RunLayout *R = new RunLayout();
+    memset((void *)R, 0, sizeof(RunLayout));
+    const int rc = build_runs(op, R);
+    if (rc != CGB_OK) {
+        drop_runs(R);
+        return rc;
+    }
+    op->runs = R;
+    return CGB_OK;
+}
+
+void free_runs(cgb_op *op) {
+    if (op->runs) drop_runs(op->runs);
+    op->runs = nullptr;
+}
+
 static void drop_plan(FfPlan *f) {
-    void *p[] = {f->run_ptr, f->run_o, f->run_seg, f->coef, f->vperm, f->fimg, f->colmax, f->aimg, f->run_blk,
-                 f->part, f->epart, f->zrow};
+    void *p[] = {f->coef, f->fimg, f->colmax, f->aimg, f->run_blk, f->part, f->epart, f->zrow};
     for (void *q : p)
         if (q) cudaFree(q);
     if (f->done) cudaEventDestroy(f->done);
@@ -993,7 +1028,7 @@ static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
 int refresh_ff_plan(cgb_op *op) {
     if (!op->ffp) return CGB_OK;
     FfPlan *f = op->ffp;
-    if (op->lut_signed || !f->run_ptr) {  // the choice of kernels changed: laid out anew
+    if (op->lut_signed || !f->colmax) {  // the choice of kernels changed: laid out anew
         free_ff_plan(op);
         return CGB_OK;
     }
@@ -1010,7 +1045,8 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     const OpDev P = op->dev();
     SmFwdArgs a;
     memset(&a, 0, sizeof(a));
-    a.vperm = f->vperm; a.run_ptr = f->run_ptr; a.run_o = f->run_o; a.coef = f->coef; a.nruns = f->nruns;
+    const RunLayout &R = *op->runs;
+    a.vperm = R.vperm; a.run_ptr = R.run_ptr; a.run_o = R.run_o; a.coef = f->coef; a.nruns = R.nruns;
     a.img = f->fimg; a.colmax = f->colmax;
     a.nIC = op->nIC; a.ndirs = op->ndirs; a.nS = op->nS; a.nc = f->fnc;
     perm_range(op, a.v0, a.v1, a.p0, a.p1);
@@ -1026,7 +1062,8 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     const bool cap = capturing(st);
     if (!cap && f->used && f->last != st) CGB_CUDA(cudaStreamWaitEvent(st, f->done, 0));
     if (op->vr1 <= 0 || op->vr0 == 0)
-        k_run_coef<<<grid_n((f->nruns + kCoefRuns - 1) / kCoefRuns), 256, 0, st>>>(P, f->run_seg, f->nruns, x, f->eval_ones, f->coef);
+        k_run_coef<<<grid_n((R.nruns + kCoefRuns - 1) / kCoefRuns), 256, 0, st>>>(P, R.run_seg, R.nruns, x, R.eval_ones,
+                                                                                  f->coef);
     CGB_CUDA(cudaGetLastError());
     const int g = sm_grid(op, f->fnc, a.p1 - a.p0, kFwdThreads / 8);
     const size_t smem = (size_t)op->nIC * op->ndirs * f->fcs * sizeof(float);
@@ -1059,8 +1096,9 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
     const OpDev P = op->dev();
     SmAdjArgs a;
     memset(&a, 0, sizeof(a));
-    a.vperm = f->vperm; a.run_blk = f->run_blk; a.run_seg = f->run_seg; a.run_o = f->run_o; a.seg_l = op->seg_l;
-    a.n = op->n; a.nruns = f->nruns; a.img = f->aimg; a.colmax = f->colmax;
+    const RunLayout &R = *op->runs;
+    a.vperm = R.vperm; a.run_blk = f->run_blk; a.run_seg = R.run_seg; a.run_o = R.run_o; a.seg_l = op->seg_l;
+    a.n = op->n; a.nruns = R.nruns; a.img = f->aimg; a.colmax = f->colmax;
     a.nIC = op->nIC; a.nS = op->nS; a.nV = op->nV; a.nc = f->anc; a.nb = f->anb; a.no = f->ano;
     perm_range(op, a.v0, a.v1, a.p0, a.p1);
     a.ec_ptr = op->ec_ptr; a.ec_col = op->ec_col; a.ec_o = op->ec_o; a.iso_ptr = op->iso_ptr; a.iso_col = op->iso_col;
@@ -1081,9 +1119,9 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
     }
     CGB_TRY(rc);
     {
-        const int64_t runs = f->nruns * (a.v1 - a.v0) / op->nV + 1;
+        const int64_t runs = R.nruns * (a.v1 - a.v0) / op->nV + 1;
         const int64_t blocks = (runs + 255) / 256, cap = (int64_t)op->nsm * 32;
-        k_adj_join<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(a, f->run_ptr);
+        k_adj_join<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(a, R.run_ptr);
         CGB_CUDA(cudaGetLastError());
     }
     *ran = 1;

@@ -28,16 +28,20 @@
 
 namespace cgb {
 
-// Run layout and table images of a handle (built on the first large float-float product)
-struct FfPlan {
-    int fwd_ok, adj_ok;          // kernels usable for this handle's shape and table
+// Runs (segments of a voxel with one orientation) of a handle, built on its first large product
+struct RunLayout {
     int64_t nruns;
     uint32_t *run_ptr;           // [nV+1] runs of voxel v
     uint16_t *run_o;             // [nruns] orientation
     uint32_t *run_seg;           // [nruns+1] first segment
-    float2 *coef;                // [nIC * nruns] run coefficients (high, low word) of the current A
     uint32_t *vperm;             // [nV] voxels, by falling run count within windows of kVoxWindow
     int eval_ones;               // eval is 1 everywhere
+};
+
+// Table images and buffers of the shared-memory float-float products
+struct FfPlan {
+    int fwd_ok, adj_ok;          // kernels usable for this handle's shape and table
+    float2 *coef;                // [nIC * nruns] run coefficients (high, low word) of the current A
     // A: samples in fnc chunks of 16 * fnp, row stride fcs floats
     int fnp, fnc, fcs;
     float *fimg;                 // [fnc][nIC * ndirs][fcs]

@@ -1,0 +1,310 @@
+// Plan, coefficient and join passes and launches of the shared-memory reduced-precision
+// products (smem_mix.cuh).
+#include <mutex>
+
+#include "smem_mix.cuh"
+
+namespace cgb {
+namespace {
+
+using namespace detail;
+
+// table image [chunk][row][cs] from rows of stride nSp, zero beyond the chunk's samples
+__global__ void k_mix_image(const unsigned short *__restrict__ lut, int rows, int nS, int nSp, int nc, int width, int cs,
+                            unsigned short *__restrict__ img) {
+    const int64_t total = (int64_t)nc * rows * cs;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(q % cs);
+        const int64_t t = q / cs;
+        const int r = (int)(t % rows), s = (int)(t / rows) * width + k;
+        img[q] = k < width && s < nS ? lut[(size_t)r * nSp + s] : (unsigned short)0;
+    }
+}
+
+__device__ __forceinline__ float mix_length(const SmMixArgs &A, uint32_t j) {
+    return __half2float(A.seg_l16[j]) * A.l_scale;
+}
+
+// run coefficients sum(l * x * eval) in FP32, four runs in flight per thread (as k_run_coef)
+__global__ void __launch_bounds__(256) k_mix_coef(const __grid_constant__ SmMixArgs A, const uint32_t *__restrict__ seg_f,
+                                                  const uint32_t *__restrict__ eval, int nF) {
+    constexpr int U = 4;
+    for (int64_t r0 = blockIdx.x * (256ll * U) + threadIdx.x; r0 < A.nruns; r0 += (int64_t)gridDim.x * (256 * U)) {
+        uint32_t beg[U], end[U], f[U];
+        float l[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t r = r0 + 256 * u < A.nruns ? r0 + 256 * u : A.nruns - 1;
+            beg[u] = A.run_seg[r];
+            end[u] = A.run_seg[r + 1];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f[u] = seg_f[beg[u]];
+            l[u] = mix_length(A, beg[u]);
+        }
+        for (int i = 0; i < A.nIC; ++i) {
+            const float *x = A.x + (size_t)i * nF;
+            const uint32_t *ev = eval ? eval + (size_t)i * nF : nullptr;
+            float c[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) c[u] = l[u] * x[f[u]] * (ev ? (float)ev[f[u]] : 1.f);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                for (uint32_t j = beg[u] + 1; j < end[u]; ++j)
+                    c[u] += mix_length(A, j) * x[seg_f[j]] * (ev ? (float)ev[seg_f[j]] : 1.f);
+                if (r0 + 256 * u < A.nruns) A.coef[(size_t)i * A.nruns + r0 + 256 * u] = c[u];
+            }
+        }
+    }
+}
+
+// several chunks: terms l * <L, z> of the segments of the voxels [v0, v1) from the runs' parts, and
+// their EC / ISO columns
+__global__ void __launch_bounds__(256) k_mix_join(const __grid_constant__ SmMixArgs A) {
+    const int64_t first = blockIdx.x * 256ll + threadIdx.x, step = gridDim.x * 256ll;
+    const int64_t r0 = A.run_ptr[A.v0], r1 = A.run_ptr[A.v1];
+    for (int64_t r = r0 + first; r < r1; r += step) {
+        const uint32_t sb = A.run_seg[r], se = A.run_seg[r + 1];
+        const float l0 = mix_length(A, sb);
+        for (int i = 0; i < A.nIC; ++i) {
+            const float *q = A.part + ((size_t)i * A.nruns + r) * A.nc;
+            float t = q[0];
+            for (int c = 1; c < A.nc; ++c) t += q[c];
+            float *out = A.scratch + (size_t)i * A.n;
+            out[sb] = l0 * t;
+            for (uint32_t g = sb + 1; g < se; ++g) out[g] = mix_length(A, g) * t;
+        }
+    }
+    auto column = [&](int64_t col) {
+        float t = A.epart[col * A.nc];
+        for (int c = 1; c < A.nc; ++c) t += A.epart[col * A.nc + c];
+        A.xout[A.ec_base + col] = (double)t;
+    };
+    if (A.nEC) {
+        const int64_t e0 = A.ec_ptr[A.v0], e1 = A.ec_ptr[A.v1];
+        for (int64_t j = e0 + first; j < e1; j += step)
+            for (int i = 0; i < A.nEC; ++i) column((int64_t)i * A.nE + A.ec_col[j]);
+    }
+    if (A.nISO) {
+        const int64_t e0 = A.iso_ptr[A.v0], e1 = A.iso_ptr[A.v1];
+        for (int64_t j = e0 + first; j < e1; j += step)
+            for (int i = 0; i < A.nISO; ++i) column(A.iso_base - A.ec_base + (int64_t)i * A.nISOv + A.iso_col[j]);
+    }
+}
+
+int grid_of(int64_t n, int cap) {
+    int64_t g = (n + 255) / 256;
+    if (g > cap) g = cap;
+    return (int)(g < 1 ? 1 : g);
+}
+
+// chunks of at most 192 samples whose table fits in a block's shared memory
+bool mix_shape(const cgb_op *op, MixPlan *m) {
+    const int64_t rows = (int64_t)op->nIC * op->ndirs;
+    for (int nc = (op->nS + 191) / 192; nc <= 8; ++nc) {
+        const int nq = (op->nS + 32 * nc - 1) / (32 * nc), cs = (32 * nq + 63) / 64 * 64;
+        if (32 * nq * (nc - 1) >= op->nS) continue;  // the last chunk would be empty
+        if (rows * cs * 2 <= (224 << 10)) {
+            m->nq = nq;
+            m->nc = nc;
+            m->cs = cs;
+            return true;
+        }
+    }
+    return false;
+}
+
+void drop(MixPlan *m) {
+    void *p[] = {m->img, m->coef, m->part, m->epart};
+    for (void *q : p)
+        if (q) cudaFree(q);
+    m->img = nullptr;
+    m->coef = m->part = m->epart = nullptr;
+}
+
+template <class T>
+int take(cgb_op *op, T **p, size_t count) {
+    CGB_CUDA(cudaMalloc((void **)p, (count ? count : 1) * sizeof(T)));
+    op->bytes += (count ? count : 1) * sizeof(T);
+    return CGB_OK;
+}
+
+int build_mix(cgb_op *op, MixPlan *m) {
+    CGB_TRY(ensure_runs(op));
+    const int64_t runs = op->runs->nruns * op->nIC;
+    CGB_TRY(take(op, &m->coef, (size_t)runs));
+    if (m->nc > 1) CGB_TRY(take(op, &m->part, (size_t)runs * m->nc));
+    if (m->nc > 1) CGB_TRY(take(op, &m->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * m->nc));
+    CGB_TRY(take(op, &m->img, (size_t)m->nc * op->nIC * op->ndirs * m->cs));
+    CGB_CUDA(cudaEventCreateWithFlags(&m->done, cudaEventDisableTiming));
+    return CGB_OK;
+}
+
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// Where these kernels take over: the size from which FP64 vectors build the same run layout, and
+// half a segment x response per voxel and chunk.  Measured (FP16, us, here / gathering kernels):
+// 6.7 M terms with 0.8 segments per voxel A 44 / 61 and A' 51 / 73, 26 M terms 30 / 50 and
+// 50 / 55, 232 M terms 68 / 122 and 104 / 155; below, the layout costs more than a few products.
+constexpr double kMixMinItems = 0.5;
+
+// the handle's plan with the image of `arith`, or null where the gathering kernels are to run.
+// Its buffers stay where they are for the handle's life: the shape does not depend on `arith`.
+int mix_plan(cgb_op *op, cudaStream_t st, int arith, MixPlan **out) {
+    *out = nullptr;
+    if (arith == CGB_ARITH_F32 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
+    if (arith == CGB_ARITH_BF16 && tc_forward_enabled(op)) return CGB_OK;
+    // an entry that is not finite, as it stands or in FP16: a zero coefficient must skip its row
+    if ((op->lut_signed & 2) || op->lut_exp_adj > (arith == CGB_ARITH_FP16 ? 14 : 126)) return CGB_OK;
+    if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork) return CGB_OK;
+    MixPlan shape{};
+    if (!mix_shape(op, &shape) || (double)op->n * op->nIC < kMixMinItems * shape.nc * op->nV) return CGB_OK;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> g(mu);
+    if (!op->mixp || (op->mixp->img && op->mixp_kind != arith)) {
+        if (capturing(st)) return CGB_OK;
+        CGB_CUDA(cudaDeviceSynchronize());
+        if (!op->mixp) {
+            MixPlan *m = new MixPlan(shape);
+            const size_t bytes = op->bytes;
+            const int rc = build_mix(op, m);
+            if (rc != CGB_OK) {
+                drop(m);
+                op->bytes = bytes;
+                if (rc != CGB_ERR_NOMEM) {
+                    delete m;
+                    return rc;
+                }
+                cudaGetLastError();  // no room: the plan stays empty and the gathering kernels run
+            }
+            op->mixp = m;
+        }
+        MixPlan *m = op->mixp;
+        if (m->img) {
+            const int rows = op->nIC * op->ndirs;
+            k_mix_image<<<grid_of((int64_t)m->nc * rows * m->cs, 4096), 256>>>(
+                (const unsigned short *)op->lut_r_ic(arith), rows, op->nS, op->nSp_r, m->nc, 32 * m->nq, m->cs, m->img);
+            CGB_CUDA(cudaGetLastError());
+            CGB_CUDA(cudaDeviceSynchronize());
+            op->mixp_kind = arith;
+        }
+    }
+    if (op->mixp->img) *out = op->mixp;
+    return CGB_OK;
+}
+
+SmMixArgs mix_args(const cgb_op *op, const MixPlan *m, int arith) {
+    const RunLayout &R = *op->runs;
+    const OpDev P = op->dev();
+    SmMixArgs a{};
+    a.vperm = R.vperm; a.run_ptr = R.run_ptr; a.run_seg = R.run_seg; a.run_o = R.run_o;
+    a.n = op->n; a.nruns = R.nruns; a.img = m->img;
+    a.nIC = op->nIC; a.ndirs = op->ndirs; a.nS = op->nS; a.nV = op->nV; a.nc = m->nc;
+    a.v0 = op->vr1 > 0 ? op->vr0 : 0;
+    a.v1 = op->vr1 > 0 ? op->vr1 : op->nV;
+    a.p0 = a.v0 / kVoxWindow * kVoxWindow;
+    a.p1 = (a.v1 + kVoxWindow - 1) / kVoxWindow * kVoxWindow;
+    if (a.p1 > op->nV) a.p1 = op->nV;
+    a.ec_ptr = op->ec_ptr; a.ec_col = op->ec_col; a.ec_o = op->ec_o; a.iso_ptr = op->iso_ptr; a.iso_col = op->iso_col;
+    a.lutEC = op->lut_r_ec(arith); a.lutISO = op->lut_r_iso(arith);
+    a.nSp = op->nSp_r;
+    a.nEC = op->nE > 0 ? op->nEC : 0; a.nISO = op->nISOv > 0 ? op->nISO : 0;
+    a.ec_base = P.ec_base; a.iso_base = P.iso_base; a.nE = op->nE; a.nISOv = op->nISOv;
+    a.seg_l16 = op->seg_l16; a.l_scale = op->len16_inv_scale;
+    a.coef = m->coef; a.part = m->part; a.epart = m->epart; a.scratch = op->scratch32;
+    return a;
+}
+
+int launch(const cgb_op *op, const MixPlan *m, int arith, int adjoint, const SmMixArgs &a, cudaStream_t st) {
+    const int need = (a.p1 - a.p0 + kMixThreads / 8 - 1) / (kMixThreads / 8);
+    int g = op->nsm / m->nc;
+    if (need < g) g = need;
+    g = m->nc * (g < 1 ? 1 : g);
+    const size_t smem = (size_t)op->nIC * op->ndirs * m->cs * 2;
+    if (arith == CGB_ARITH_BF16) return launch_mix_smem_bf16(adjoint, m->nq, g, smem, st, a, m->cs);
+    return launch_mix_smem_fp16(adjoint, m->nq, g, smem, st, a, m->cs);
+}
+
+// the buffers belong to the handle: a product on another stream waits for the last one (under
+// capture the graph's own order applies)
+int enter(MixPlan *m, cudaStream_t st) {
+    if (!capturing(st) && m->used && m->last != st) CGB_CUDA(cudaStreamWaitEvent(st, m->done, 0));
+    return CGB_OK;
+}
+int leave(MixPlan *m, cudaStream_t st) {
+    if (capturing(st)) return CGB_OK;
+    CGB_CUDA(cudaEventRecord(m->done, st));
+    m->last = st;
+    m->used = 1;
+    return CGB_OK;
+}
+
+}  // namespace
+
+void free_mix_plan(cgb_op *op) {
+    if (!op->mixp) return;
+    drop(op->mixp);
+    if (op->mixp->done) cudaEventDestroy(op->mixp->done);
+    delete op->mixp;
+    op->mixp = nullptr;
+}
+
+int forward_smem_mix(cgb_op *op, const float *x, float *y, cudaStream_t st, int arith, int *ran) {
+    *ran = 0;
+    CGB_TRY(ensure_reduced(op, arith));
+    MixPlan *m;
+    CGB_TRY(mix_plan(op, st, arith, &m));
+    if (!m) return CGB_OK;
+    SmMixArgs a = mix_args(op, m, arith);
+    a.x = x;
+    a.y = y;
+    a.vec_ok = op->nS % 4 == 0 && (uintptr_t)y % 16 == 0;
+    CGB_TRY(enter(m, st));
+    k_mix_coef<<<grid_of((a.nruns + 3) / 4, 8192), 256, 0, st>>>(a, op->seg_f, op->runs->eval_ones ? nullptr : op->eval, op->nF);
+    CGB_CUDA(cudaGetLastError());
+    CGB_TRY(launch(op, m, arith, 0, a, st));
+    CGB_TRY(leave(m, st));
+    *ran = 1;
+    return CGB_OK;
+}
+
+int adjoint_smem_mix(cgb_op *op, const float *y, double *x, cudaStream_t st, int arith, int *ran) {
+    *ran = 0;
+    CGB_TRY(ensure_reduced(op, arith));
+    MixPlan *m;
+    CGB_TRY(mix_plan(op, st, arith, &m));
+    if (!m) return CGB_OK;
+    CGB_TRY(enter(m, st));
+    auto pass = [&](cudaStream_t q) -> int {
+        SmMixArgs a = mix_args(op, m, arith);
+        a.z = y;
+        a.xout = x;
+        a.vec_ok = op->nS % 4 == 0 && (uintptr_t)y % 16 == 0;
+        CGB_TRY(launch(op, m, arith, 1, a, q));
+        if (m->nc == 1) return CGB_OK;
+        k_mix_join<<<grid_of(a.nruns * (a.v1 - a.v0) / op->nV + 1, op->nsm * 32), 256, 0, q>>>(a);
+        CGB_CUDA(cudaGetLastError());
+        return CGB_OK;
+    };
+    if (op->nslab <= 1) {
+        CGB_TRY(pass(st));
+        CGB_TRY(fibre_sum32_from(op, op->scratch32, x, st));
+    } else {
+        CGB_TRY(slab_schedule(
+            op, st,
+            [&](int s, cudaStream_t q) {
+                VoxelRange vr(op, op->slab_v[s], op->slab_v[s + 1]);
+                return pass(q);
+            },
+            [&](int s, cudaStream_t q) { return fibre_sum32_slab(op, op->scratch32, x, s, q); }));
+    }
+    CGB_TRY(leave(m, st));
+    *ran = 1;
+    return CGB_OK;
+}
+
+}  // namespace cgb
