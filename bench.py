@@ -316,11 +316,12 @@ def launches_per_pair(A, reduced: bool, tc: bool = False) -> int:
     """Kernels of one A + A' pair.  FP64 path: the max-|x| pass of the range guard and the
     forward (large operators: the run coefficients before it), then per adjoint slab a voxel
     pass (large operators: the join of its parts) and a fibre pass.  Reduced precision: the
-    FP32 -> FP64 column conversion and the forward, the adjoint (slab passes, or the
-    tensor-core voxel pass and its fibre pass) and the FP64 -> FP32 conversion; the
-    tensor-core forward adds its x*eval pass."""
+    FP32 -> FP64 column conversion (large operators: the run coefficients) and the forward,
+    the adjoint (slab passes, or the tensor-core voxel pass and its fibre pass) and the
+    FP64 -> FP32 conversion; the tensor-core forward, taken from seven 32-sample blocks x
+    responses on, adds its x*eval pass."""
     ns = max(1, A.set_slabs(None))
-    if tc:
+    if tc and A.ICnRF * -(-A.nSAMPLES // 32) > 6:
         return 3 + 3
     if reduced:
         return 2 + 2 * ns + 1

@@ -151,18 +151,28 @@ bool capturing(cudaStream_t st) {
 // 6.7 M terms with 0.8 segments per voxel A 44 / 61 and A' 51 / 73, 26 M terms 30 / 50 and
 // 50 / 55, 232 M terms 68 / 122 and 104 / 155; below, the layout costs more than a few products.
 constexpr double kMixMinItems = 0.5;
+// Against the tensor-core kernels (BF16), whose time hardly depends on the samples but grows with
+// every segment, where this one follows the runs and the quads of samples: A here up to 6 quads x
+// responses, A' up to 4, and up to 6 from 300 segments per voxel on.  Measured (us, here / tensor
+// cores): 10 M segments, 200 per voxel: 145 samples (5 quads) A 204 / 249 and A' 297 / 304, 280
+// samples (10) 314 / 255 and 467 / 367; 184 per voxel, 145 samples A 977 / 1188 and A'
+// 1503 / 1420; 598 per voxel 406 / 541 and 693 / 950; 176 per voxel, 99 samples (4) 1396 / 1830
+// and 2211 / 2348; three responses (15) 415 / 383 and 599 / 441.
+constexpr int64_t kTcAdjDense = 300;
 
 // the handle's plan with the image of `arith`, or null where the gathering kernels are to run.
 // Its buffers stay where they are for the handle's life: the shape does not depend on `arith`.
-int mix_plan(cgb_op *op, cudaStream_t st, int arith, MixPlan **out) {
+int mix_plan(cgb_op *op, cudaStream_t st, int arith, int adjoint, MixPlan **out) {
     *out = nullptr;
     if (arith == CGB_ARITH_F32 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
-    if (arith == CGB_ARITH_BF16 && tc_forward_enabled(op)) return CGB_OK;
+    const bool tc = arith == CGB_ARITH_BF16 && tc_forward_enabled(op);
+    if (tc && op->tc_mode == 2) return CGB_OK;
     // an entry that is not finite, as it stands or in FP16: a zero coefficient must skip its row
     if ((op->lut_signed & 2) || op->lut_exp_adj > (arith == CGB_ARITH_FP16 ? 14 : 126)) return CGB_OK;
     if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork) return CGB_OK;
     MixPlan shape{};
     if (!mix_shape(op, &shape) || (double)op->n * op->nIC < kMixMinItems * shape.nc * op->nV) return CGB_OK;
+    if (tc && op->nIC * shape.nc * shape.nq > (adjoint && op->n < kTcAdjDense * op->nV ? 4 : 6)) return CGB_OK;
     static std::mutex mu;
     std::lock_guard<std::mutex> g(mu);
     if (!op->mixp || (op->mixp->img && op->mixp_kind != arith)) {
@@ -257,7 +267,7 @@ int forward_smem_mix(cgb_op *op, const float *x, float *y, cudaStream_t st, int 
     *ran = 0;
     CGB_TRY(ensure_reduced(op, arith));
     MixPlan *m;
-    CGB_TRY(mix_plan(op, st, arith, &m));
+    CGB_TRY(mix_plan(op, st, arith, 0, &m));
     if (!m) return CGB_OK;
     SmMixArgs a = mix_args(op, m, arith);
     a.x = x;
@@ -276,7 +286,7 @@ int adjoint_smem_mix(cgb_op *op, const float *y, double *x, cudaStream_t st, int
     *ran = 0;
     CGB_TRY(ensure_reduced(op, arith));
     MixPlan *m;
-    CGB_TRY(mix_plan(op, st, arith, &m));
+    CGB_TRY(mix_plan(op, st, arith, 1, &m));
     if (!m) return CGB_OK;
     CGB_TRY(enter(m, st));
     auto pass = [&](cudaStream_t q) -> int {

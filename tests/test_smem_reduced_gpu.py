@@ -49,3 +49,27 @@ def test_products_match_the_oracle(arith, nS, n_fibers, ndirs, nIC, nEC, nISO, s
         for g, e, scale in zip(got[0], exact, ref):
             assert np.all(np.abs(g - e) <= TOL[arith] * scale + 1e-30)
         assert not np.array_equal(got[0][0], got[1][0])  # the kernels under test ran
+
+
+@pytest.mark.parametrize('nS,nIC,n_fibers,dim,fwd,adj', [
+    (128, 1, 3000, (14, 14, 14), True, True), (129, 1, 2500, (14, 14, 14), True, False),
+    (129, 1, 16000, (14, 14, 14), True, True), (192, 1, 12000, (14, 14, 14), True, True),
+    (193, 1, 12000, (14, 14, 14), False, False), (97, 2, 8000, (14, 14, 14), False, False)])
+def test_bf16_choice_against_the_tensor_cores(nS, nIC, n_fibers, dim, fwd, adj):
+    """The automatic choice is the shared-memory kernel (tensor cores off) or the tensor-core one
+    (always on) by quads of samples x responses and segments per voxel."""
+    from commit_gb300.operator import LinearOperator
+    D, K = _problem(nS, n_fibers, n_mask=900, dim=dim, ndirs=120, nIC=nIC)
+    rng = np.random.default_rng(1)
+    got = []
+    for mode in (0, 1, 2):
+        A = LinearOperator(D, K, None)
+        A.tensor_cores(mode)
+        if mode == 0:
+            assert A.tensor_cores() == 1
+            x = torch.from_numpy(rng.uniform(0, 1, A.nCOLS).astype(np.float32)).cuda()
+            y = torch.from_numpy(rng.uniform(0, 1, A.nROWS).astype(np.float32)).cuda()
+        got.append((A.dot(x, arith='bf16'), A.T.dot(y, arith='bf16')))
+    for k, smem in ((0, fwd), (1, adj)):
+        assert torch.equal(got[0][k], got[1 if smem else 2][k])
+        assert not torch.equal(got[1][k], got[2][k])
