@@ -140,6 +140,7 @@ int cgb_op_apply(cgb_op *op, int adjoint, const void *in, int64_t in_len, void *
     DevGuard g(op->device);
     cudaStream_t st = (cudaStream_t)stream;
     if (out_len == 0) return CGB_OK;
+    InPlaceScope in_place(st);
     if (dtype == CGB_DTYPE_F64) {
         const int ar = (arith == CGB_ARITH_F64 || arith == CGB_ARITH_FF) ? arith : op->arith;
         if (in_len == 0) {

@@ -197,6 +197,15 @@ int launch_resnorm_grid(cgb_op *op, const double *x, const double *y, const doub
 int launch_gradient_grid(cgb_op *op, const double *x, const double *y, const double *sqw, double *grad,
                          double *partials, const double *ax_a, const double *ax_b, double ca, double cb,
                          cudaStream_t st, int arith, int *grid);
+// While one lives, this thread's products keep to the kernels that read the handle's tables in
+// place: a caller's captured graph may be replayed after the table is replaced, when the layouts
+// and the choice of kernels made from the old table no longer hold.
+struct InPlaceScope {
+    explicit InPlaceScope(cudaStream_t st);
+    ~InPlaceScope();
+    bool was;
+};
+bool in_place_only();
 // float-float products with the table in shared memory (smem_ff.cu)
 int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const double *yobs, const double *sqw,
                  double *partials, cudaStream_t st, int *grid, int *ran);

@@ -959,6 +959,11 @@ int launch_sm(F kern, int grid, int threads, size_t smem, cudaStream_t st, const
 
 }  // namespace
 
+static thread_local bool in_place = false;
+InPlaceScope::InPlaceScope(cudaStream_t st) : was(in_place) { in_place = in_place || capturing(st); }
+InPlaceScope::~InPlaceScope() { in_place = was; }
+bool in_place_only() { return in_place; }
+
 // the handle's runs, laid out on first use (not under stream capture: the callers see to it)
 int ensure_runs(cgb_op *op) {
     static std::mutex m;
@@ -998,7 +1003,7 @@ void free_ff_plan(cgb_op *op) {
 // the handle's plan if the shared-memory kernels are to run this product, else null
 static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
     *out = nullptr;
-    if (op->ff_variant != 1 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
+    if (in_place_only() || op->ff_variant != 1 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
     if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork) return CGB_OK;
     if (!op->ffp) {
         if (capturing(st)) return CGB_OK;

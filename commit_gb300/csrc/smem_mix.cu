@@ -141,11 +141,6 @@ int build_mix(cgb_op *op, MixPlan *m) {
     return CGB_OK;
 }
 
-bool capturing(cudaStream_t st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
-}
-
 // Where these kernels take over: the size from which FP64 vectors build the same run layout, and
 // half a segment x response per voxel and chunk.  Measured (FP16, us, here / gathering kernels):
 // 6.7 M terms with 0.8 segments per voxel A 44 / 61 and A' 51 / 73, 26 M terms 30 / 50 and
@@ -164,7 +159,7 @@ constexpr int64_t kTcAdjDense = 300;
 // Its buffers stay where they are for the handle's life: the shape does not depend on `arith`.
 int mix_plan(cgb_op *op, cudaStream_t st, int arith, int adjoint, MixPlan **out) {
     *out = nullptr;
-    if (arith == CGB_ARITH_F32 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
+    if (in_place_only() || arith == CGB_ARITH_F32 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
     const bool tc = arith == CGB_ARITH_BF16 && tc_forward_enabled(op);
     if (tc && op->tc_mode == 2) return CGB_OK;
     // an entry that is not finite, as it stands or in FP16: a zero coefficient must skip its row
@@ -176,7 +171,6 @@ int mix_plan(cgb_op *op, cudaStream_t st, int arith, int adjoint, MixPlan **out)
     static std::mutex mu;
     std::lock_guard<std::mutex> g(mu);
     if (!op->mixp || (op->mixp->img && op->mixp_kind != arith)) {
-        if (capturing(st)) return CGB_OK;
         CGB_CUDA(cudaDeviceSynchronize());
         if (!op->mixp) {
             MixPlan *m = new MixPlan(shape);
@@ -239,14 +233,12 @@ int launch(const cgb_op *op, const MixPlan *m, int arith, int adjoint, const SmM
     return launch_mix_smem_fp16(adjoint, m->nq, g, smem, st, a, m->cs);
 }
 
-// the buffers belong to the handle: a product on another stream waits for the last one (under
-// capture the graph's own order applies)
+// the buffers belong to the handle: a product on another stream waits for the last one
 int enter(MixPlan *m, cudaStream_t st) {
-    if (!capturing(st) && m->used && m->last != st) CGB_CUDA(cudaStreamWaitEvent(st, m->done, 0));
+    if (m->used && m->last != st) CGB_CUDA(cudaStreamWaitEvent(st, m->done, 0));
     return CGB_OK;
 }
 int leave(MixPlan *m, cudaStream_t st) {
-    if (capturing(st)) return CGB_OK;
     CGB_CUDA(cudaEventRecord(m->done, st));
     m->last = st;
     m->used = 1;

@@ -121,6 +121,39 @@ def test_table_signs_and_new_tables():
         assert G.rel(B.dot(x), P.dot(x)) <= TOL and G.rel(B.T.dot(y), P.T.dot(y)) <= TOL
 
 
+def test_captured_products_follow_the_table():
+    """A caller's graph of A and A', captured before and after the layout exists, gives the
+    products of the table in place when it is replayed, also one with other signs."""
+    import ctypes
+    from commit_gb300._lib import check, lib
+    from commit_gb300.operator import LinearOperator
+    D, K = _problem(97, 6000)
+    A = LinearOperator(D, K, None)
+    rng = np.random.default_rng(8)
+    x, y = rng.uniform(0, 1, A.nCOLS), rng.uniform(0, 1, A.nROWS)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    graphs = []
+    for _ in range(2):
+        ax, aty = torch.empty_like(yd), torch.empty_like(xd)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            A.dot(xd, out=ax)
+            A.T.dot(yd, out=aty)
+        graphs.append((g, ax, aty))
+        A.dot(xd), A.T.dot(yd)
+    for sign in (1.0, -1.0):
+        K2 = dict(K, wmr=(K['wmr'] * rng.uniform(0.5, 1.0, K['wmr'].shape)).astype(np.float32))
+        K2['wmr'][0, 0::2] *= sign
+        check(lib().cgb_op_set_lut(A.handle, K2['wmr'].ctypes.data_as(ctypes.c_void_p), None, None))
+        P = O.PortOperator(D, K2, None, nthreads=8)
+        rx, ry = P.dot(x), P.T.dot(y)
+        for g, ax, aty in graphs:
+            g.replay()
+            torch.cuda.synchronize()
+            assert G.rel(ax.cpu().numpy(), rx) <= TOL and G.rel(aty.cpu().numpy(), ry) <= TOL
+
+
 @pytest.mark.parametrize('bad', [np.inf, -np.inf, np.nan])
 def test_non_finite_input_stays_in_its_voxels(bad):
     D, K = _problem(97, 6000)
