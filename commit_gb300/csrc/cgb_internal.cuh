@@ -172,8 +172,8 @@ struct cgb_op {
     __nv_bfloat16 *tc_rows16;       // EC rows (nEC * ndirs) then ISO rows (nISO) as BF16, stride tc_np
     int lut_signed;                 // bit 0: an IC table value is negative or not finite, bit 1: any table value is not finite
     cgb::RunLayout *runs;           // built on the first product that uses them
-    cgb::MixPlan *mixp;             // buffers of the FP32-vector products, likewise
-    int mixp_kind;                  // arithmetic of its table image (0: to be filled)
+    cgb::MixPlan *mixp[2];          // buffers of the FP32-vector products (16-bit, FP32 table), likewise
+    int mixp_kind[2];               // arithmetic of their table images (0: to be filled)
     cgb::FfPlan *ffp;               // run layout of the shared-memory products, built on first use
     int ff_pinned;                  // a build or shape of the pair kernels was set: they run
     size_t bytes;

@@ -580,7 +580,7 @@ int cgb_op_set_lut(cgb_op *op, const float *lutIC, const float *lutEC, const flo
                               cudaMemcpyDefault));
     }
     op->lut_r_kind = 0;  // reduced-precision copies are rebuilt on their next use
-    op->mixp_kind = 0;
+    op->mixp_kind[0] = op->mixp_kind[1] = 0;
     CGB_TRY(update_lut_exponents(op));
     return refresh_ff_plan(op);
 }

@@ -4,13 +4,14 @@
 // coefficients of a batch (scans, shuffles) and on rows of two voxels per warp; keeping their
 // structure and only moving the table to shared memory gained nothing (measured).  Here the
 // runs (smem_ff.cuh) get their coefficients in one pass, a warp takes four voxels, 8 lanes and
-// four samples per load each, and the BF16 or FP16 table stays in shared memory for the
-// launch, in chunks of the samples where it does not fit.  FP32 accumulation
+// four samples per load each, and the table (BF16, FP16 or FP32) stays in shared memory for
+// the launch, in chunks of the samples where it does not fit.  FP32 accumulation
 // and FP16 lengths as in the gathering kernels; only the order of the sums differs, so the
 // solvers (whose FP64 iterates would show it) stay on those, and FP32 products come here.
-// The passes are bound by the conversions and FMAs of the runs (a quad costs two 16-bit to FP32
+// The passes are bound by the conversions and FMAs of the runs (a quad of 16-bit values costs two
 // conversions and two packed FMAs for its one load).  Measured on a tractogram of 15 M segments x
-// 145 samples (FP16): A 693 -> 298 us and 78 for the coefficients, A' 842 -> 395 us.
+// 145 samples: FP16 A 693 -> 298 us and 78 for the coefficients, A' 842 -> 395 us; FP32 (two
+// chunks) A 679 -> 559 us in all and A' 975 -> 764.
 #pragma once
 #include "operator_mixed.cuh"
 #include "smem_ff.cuh"
@@ -19,10 +20,10 @@ namespace cgb {
 
 struct MixPlan {
     int nq, nc, cs;      // quads of samples per lane, chunks of 32 * nq samples, row stride (elements)
-    unsigned short *img; // [nc][nIC * ndirs][cs] (null: no room for the buffers)
+    char *img;           // [nc][nIC * ndirs][cs] (null: no room for the buffers)
     float *coef;         // [nIC * nruns]
     float *part;         // [nIC * nruns][nc] (nc > 1)
-    float *epart;        // [EC and ISO columns][nc] (nc > 1)
+    double *epart;       // [EC and ISO columns][nc] (nc > 1)
     cudaEvent_t done;    // the last product has finished with the buffers
     cudaStream_t last;   // ... and its stream
     int used;
@@ -46,6 +47,20 @@ struct Quad {
         conv(__ldg(reinterpret_cast<const uint2 *>(p)), a, b);
     }
 };
+template <>
+struct Quad<float> {
+    __device__ static __forceinline__ void lds(const float *p, f2 &a, f2 &b) {
+        const ulonglong2 u = *reinterpret_cast<const ulonglong2 *>(p);
+        a = u.x;
+        b = u.y;
+    }
+    __device__ static __forceinline__ void ldg(const float *p, f2 &a, f2 &b) {
+        const ulonglong2 u = __ldg(reinterpret_cast<const ulonglong2 *>(p));
+        a = u.x;
+        b = u.y;
+    }
+};
+
 struct SmMixArgs {
     const uint32_t *vperm, *run_ptr, *run_seg;
     const uint16_t *run_o;
@@ -61,17 +76,33 @@ struct SmMixArgs {
     float *y;                    // A: rows
     const float *z;              // A': rows
     double *xout;                // A': columns
-    const __half *seg_l16;       // lengths times 1 / l_scale
+    const __half *seg_l16;       // lengths times 1 / l_scale (FP32 table: null, and seg_l)
+    const float *seg_l;
     float l_scale;
-    float *coef, *part, *epart, *scratch;
+    float *coef, *part, *scratch;
+    double *epart;
     int vec_ok;                  // rows are 16-byte aligned and a multiple of four samples
 };
 
-// quad of register k: odd groups take neighbouring quads swapped (rows are a multiple of 128
+template <bool F32>
+__device__ __forceinline__ float mix_length(const SmMixArgs &A, uint32_t j) {
+    return F32 ? A.seg_l[j] : __half2float(A.seg_l16[j]) * A.l_scale;
+}
+
+// a + b in s with its rounding error in e (0 when the sum is not finite): with an FP32 table the
+// last sums of a dot product are those that show, and the term l * (s + e) rounds once
+__device__ __forceinline__ float sum_err(float a, float b, float &e) {
+    const float s = a + b, bb = s - a;
+    e = (a - (s - bb)) + (b - bb);
+    if (!(fabsf(e) <= 3.0e38f)) e = 0.f;
+    return s;
+}
+
+// quad of register k: odd groups take neighbouring quads swapped (16-bit rows are a multiple of 128
 // bytes apart, and the two groups of a half-warp then read the two halves of a line)
-template <int NQ>
+template <class LT, int NQ>
 __device__ __forceinline__ int quad_of(int k, int par) {
-    return (k ^ 1) < NQ ? k ^ par : k;
+    return sizeof(LT) == 2 && (k ^ 1) < NQ ? k ^ par : k;
 }
 
 template <class LT, int NQ>
@@ -81,7 +112,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_fwd_mix_smem(const __grid_co
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane & 7, lg = lane >> 3, par = lg & 1;
     const int chunk = blockIdx.x % A.nc, cta = blockIdx.x / A.nc, ncta = gridDim.x / A.nc;
-    const int rows = A.nIC * A.ndirs, words = rows * cs / 2;
+    const int rows = A.nIC * A.ndirs, words = rows * cs * (int)sizeof(LT) / 4;
     fill_table<kMixThreads>(smraw, reinterpret_cast<const float *>(A.img) + (size_t)chunk * words, words);
     const int s_base = chunk * 32 * NQ;
     const int last = A.p1 - A.p0, stride = ncta * (kMixThreads / 8);
@@ -112,7 +143,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_fwd_mix_smem(const __grid_co
 #pragma unroll
             for (int k = 0; k < NQ; ++k) {
                 f2 u, t;
-                Quad<LT>::lds(L + 32 * quad_of<NQ>(k, par), u, t);
+                Quad<LT>::lds(L + 32 * quad_of<LT, NQ>(k, par), u, t);
                 a0[k] = f2_fma(c2, u, a0[k]);
                 a1[k] = f2_fma(c2, t, a1[k]);
             }
@@ -178,7 +209,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_fwd_mix_smem(const __grid_co
                 const f2 c2 = f2_pack(ct, ct);
 #pragma unroll
                 for (int k = 0; k < NQ; ++k) {
-                    const int o = 32 * quad_of<NQ>(k, par);
+                    const int o = 32 * quad_of<LT, NQ>(k, par);
                     if (s_base + o + 4 * sub < A.nSp) {
                         f2 u, s;
                         Quad<LT>::ldg(L + o, u, s);
@@ -191,7 +222,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_fwd_mix_smem(const __grid_co
         if (v >= 0) {
 #pragma unroll
             for (int k = 0; k < NQ; ++k) {
-                const int s = s_base + 4 * (sub + 8 * quad_of<NQ>(k, par));
+                const int s = s_base + 4 * (sub + 8 * quad_of<LT, NQ>(k, par));
                 if (s >= A.nS) continue;
                 float o[4];
                 f2_unpack(a0[k], o[0], o[1]);
@@ -222,7 +253,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_adj_mix_smem(const __grid_co
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane & 7, lg = lane >> 3, par = lg & 1;
     const int chunk = blockIdx.x % A.nc, cta = blockIdx.x / A.nc, ncta = gridDim.x / A.nc;
-    const int rows = A.nIC * A.ndirs, words = rows * cs / 2;
+    const int rows = A.nIC * A.ndirs, words = rows * cs * (int)sizeof(LT) / 4;
     fill_table<kMixThreads>(smraw, reinterpret_cast<const float *>(A.img) + (size_t)chunk * words, words);
     const int s_base = chunk * 32 * NQ;
     const int last = A.p1 - A.p0, stride = ncta * (kMixThreads / 8);
@@ -251,7 +282,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_adj_mix_smem(const __grid_co
         f2 z0[NQ], z1[NQ];
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
-            const int s = s_base + 4 * (sub + 8 * quad_of<NQ>(k, par));
+            const int s = s_base + 4 * (sub + 8 * quad_of<LT, NQ>(k, par));
             float o[4] = {0.f, 0.f, 0.f, 0.f};
             if (v >= 0 && s < A.nS) {
                 const float *p = A.z + (size_t)v * A.nS + s;
@@ -288,7 +319,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_adj_mix_smem(const __grid_co
             const bool okn = jn < (b + 8 < most ? re : ren);
             on = okn ? __ldg(A.run_o + jn) : 0u;
             const uint32_t sb = sn, se = en;
-            const float l0 = whole && valid ? __half2float(A.seg_l16[sb]) * A.l_scale : 0.f;
+            const float l0 = whole && valid ? mix_length<sizeof(LT) == 4>(A, sb) : 0.f;
             segs(jn, okn);
 #pragma unroll 1
             for (int i = 0; i < A.nIC; ++i) {
@@ -304,13 +335,16 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_adj_mix_smem(const __grid_co
                     for (int q = 0; q < 4; ++q) {
                         const LT *L = tab + __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8) + 4 * sub;
                         P[q] = 0ull;
+                        f2 R = 0ull;  // FP32 table: two chains, the rounding of a chain grows with its length
 #pragma unroll
                         for (int k = 0; k < NQ; ++k) {
                             f2 a, c;
-                            Quad<LT>::lds(L + 32 * quad_of<NQ>(k, par), a, c);
+                            Quad<LT>::lds(L + 32 * quad_of<LT, NQ>(k, par), a, c);
                             P[q] = f2_fma(a, z0[k], P[q]);
-                            P[q] = f2_fma(c, z1[k], P[q]);
+                            if (sizeof(LT) == 4) R = f2_fma(c, z1[k], R);
+                            else P[q] = f2_fma(c, z1[k], P[q]);
                         }
+                        if (sizeof(LT) == 4) P[q] = f2_add(P[q], R);
                     }
 #pragma unroll
                     for (int h = 2, d = 4; h >= 1; h /= 2, d /= 2)
@@ -325,8 +359,13 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_adj_mix_smem(const __grid_co
                 if (!valid) continue;
                 if (whole) {
                     float *out = A.scratch + (size_t)i * A.n;
-                    out[sb] = l0 * (t0 + t1);
-                    for (uint32_t g = sb + 1; g < se; ++g) out[g] = __half2float(A.seg_l16[g]) * A.l_scale * (t0 + t1);
+                    float e = 0.f;
+                    const float t = sizeof(LT) == 4 ? sum_err(t0, t1, e) : t0 + t1;
+                    out[sb] = fmaf(l0, t, l0 * e);
+                    for (uint32_t g = sb + 1; g < se; ++g) {
+                        const float l = mix_length<sizeof(LT) == 4>(A, g);
+                        out[g] = fmaf(l, t, l * e);
+                    }
                 } else {
                     A.part[((size_t)i * A.nruns + j) * A.nc + chunk] = t0 + t1;
                 }
@@ -363,31 +402,45 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_adj_mix_smem(const __grid_co
                 col = A.iso_base - A.ec_base + (int64_t)i * A.nISOv + A.iso_col[ib + (q - te) / A.nISO];
             }
             const int cnt = min(m - b, 8);
-            float mine = 0.f;
+            double mine = 0.0;
 #pragma unroll 1
             for (int t = 0; t < cnt; ++t) {
                 const LT *L = reinterpret_cast<const LT *>(
                                   __shfl_sync(full, reinterpret_cast<unsigned long long>(row), t, 8)) + s_base + 4 * sub;
-                f2 P = 0ull;
+                f2 P = 0ull, R = 0ull;
 #pragma unroll
                 for (int k = 0; k < NQ; ++k) {
-                    const int o = 32 * quad_of<NQ>(k, par);
+                    const int o = 32 * quad_of<LT, NQ>(k, par);
                     if (s_base + o + 4 * sub < A.nSp) {
                         f2 a, c;
                         Quad<LT>::ldg(L + o, a, c);
                         P = f2_fma(a, z0[k], P);
-                        P = f2_fma(c, z1[k], P);
+                        R = f2_fma(c, z1[k], R);
                     }
                 }
+                P = f2_add(P, R);
+                float t0, t1, e = 0.f;
+                if (sizeof(LT) == 4) {  // single dots: the last three sums keep their errors
+                    P = f2_add(P, __shfl_xor_sync(full, P, 4, 8));
+                    f2_unpack(P, t0, t1);
+                    t0 = sum_err(t0, t1, e);
 #pragma unroll
-                for (int d = 4; d >= 1; d >>= 1) P = f2_add(P, __shfl_xor_sync(full, P, d, 8));
-                float t0, t1;
-                f2_unpack(P, t0, t1);
-                if (sub == t) mine = t0 + t1;
+                    for (int d = 2; d >= 1; d >>= 1) {
+                        float g;
+                        t0 = sum_err(t0, __shfl_xor_sync(full, t0, d, 8), g);
+                        e += __shfl_xor_sync(full, e, d, 8) + g;
+                    }
+                    t1 = 0.f;
+                } else {
+#pragma unroll
+                    for (int d = 4; d >= 1; d >>= 1) P = f2_add(P, __shfl_xor_sync(full, P, d, 8));
+                    f2_unpack(P, t0, t1);
+                }
+                if (sub == t) mine = sizeof(LT) == 4 ? (double)t0 + (double)e : (double)(t0 + t1);
             }
             if (col >= 0) {
                 if (A.nc > 1) A.epart[col * A.nc + chunk] = mine;
-                else A.xout[A.ec_base + col] = (double)mine;
+                else A.xout[A.ec_base + col] = mine;
             }
         }
         __syncwarp();
@@ -419,5 +472,6 @@ int launch_mix_smem(int adjoint, int nq, int grid, size_t smem, cudaStream_t st,
 
 int launch_mix_smem_bf16(int adjoint, int nq, int grid, size_t smem, cudaStream_t st, const detail::SmMixArgs &a, int cs);
 int launch_mix_smem_fp16(int adjoint, int nq, int grid, size_t smem, cudaStream_t st, const detail::SmMixArgs &a, int cs);
+int launch_mix_smem_f32(int adjoint, int nq, int grid, size_t smem, cudaStream_t st, const detail::SmMixArgs &a, int cs);
 
 }  // namespace cgb

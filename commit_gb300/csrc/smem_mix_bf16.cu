@@ -1,4 +1,4 @@
-// The shared-memory reduced-precision kernels with a bf16 table (smem_mix.cuh).
+// The shared-memory reduced-precision kernels with a BF16 table (smem_mix.cuh).
 #include "smem_mix.cuh"
 
 namespace cgb {

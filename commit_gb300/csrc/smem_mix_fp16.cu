@@ -1,4 +1,4 @@
-// The shared-memory reduced-precision kernels with a fp16 table (smem_mix.cuh).
+// The shared-memory reduced-precision kernels with an FP16 table (smem_mix.cuh).
 #include "smem_mix.cuh"
 
 namespace cgb {
