@@ -73,7 +73,7 @@ __device__ __forceinline__ void block_sum_store_n(double (&v)[NV], double *dst) 
 // Warp sums of NV values at once by a butterfly reduce-scatter: lane l is left with the total of
 // value l / (32 / NV).  NV = 4 takes 6 FP64 additions per lane instead of 20 -- the pipe runs at 2
 // lanes / clock / SM, and the block sums of the statistics were most of their kernels' time
-// (k_stats on 480k columns 26 -> 11 us, k_prox_stats on 65k 25.6 -> 9).
+// (k_stats on 480k columns 26 -> 12.7 us, k_prox_stats on 65k 25.6 -> 10.5).
 template <int NV>
 __device__ __forceinline__ double warp_scatter_sum(double (&v)[NV]) {
     const int lane = threadIdx.x & 31;

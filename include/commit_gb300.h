@@ -220,11 +220,12 @@ int cgb_op_adjoint_noalloc(int nS, int ndirs, int nF, int64_t n, int nE, int nV,
  * the shape allows it (an IC compartment, nS <= 320, fewer than 2^26 columns) and the IC
  * segments are dense enough for the dense product to pay, at least 32 per voxel on
  * average (measured on GB300: 1.5x faster than the CUDA-core kernels at 62 per voxel,
- * 1.9x at 212, slower at 21); 1 keeps the CUDA-core kernels; 2 requires it
- * (CGB_ERR_UNSUPPORTED when the shape does not allow it); a negative mode only reads.
- * *out (may be NULL) receives 1 when the tensor-core kernels are in use.  The first use on
- * a handle builds its tile-ordered entry stream and LUT images (about 6 bytes per
- * segment).  No counterpart in the reference (setup_operator.py:50-218 and 591-710 are its
+ * 1.9x at 212, slower at 21); products of FP32 vectors with up to 192 samples and one
+ * response then still run on the CUDA cores where their runs cost less; 1 keeps the
+ * CUDA-core kernels; 2 requires it (CGB_ERR_UNSUPPORTED when the shape does not allow it);
+ * a negative mode only reads.  *out (may be NULL) receives 1 when the tensor-core kernels
+ * are chosen by the shape and density rules.  The first use on a handle builds its
+ * tile-ordered entry stream and LUT images (about 6 bytes per segment).  No counterpart in the reference (setup_operator.py:50-218 and 591-710 are its
  * CPU A and A').
  */
 int cgb_op_tensor_cores(cgb_op *op, int mode, int *out);
