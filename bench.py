@@ -32,11 +32,11 @@ METRIC = 'A·x+Aᵀx operator pairs/s (1M-streamline workload)'
 
 # DRAM bytes (read + write) per product, recorded from one ncu capture of this workload
 # (`ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum
-# --clock-control none -k regex:"k_(forward_p|adjoint_p|fibre_sum)" --csv python bench.py
+# --clock-control none -k regex:"k_(run_coef|fwd_smem|adj_smem|adj_join|fibre_pass)" --csv python bench.py
 # --steps 1 --warmup 1 --no-e2e --no-cpu`, one pass, full workload).  A constant: the bench
-# line labels it as such.  Keyed by (workload, streamlines, arith); the A' entry is the slab
-# voxel passes plus the slab fibre passes of one product.
-MEASURED_TRAFFIC = {('hcp_1m', 1000000, 'ff'): {'forward': 2679165952, 'adjoint': 11855011840}}
+# line labels it as such.  Keyed by (workload, streamlines, arith); the A entry is the run
+# coefficients and the voxel pass, the A' entry the slabs' voxel, join and fibre passes.
+MEASURED_TRAFFIC = {('hcp_1m', 1000000, 'ff'): {'forward': 4424852224, 'adjoint': 16377132032}}
 
 
 # relative-error bounds of the reduced-precision LUT formats (the FP64 path's bar is 1e-10)
