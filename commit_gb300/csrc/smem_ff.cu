@@ -1037,7 +1037,10 @@ int refresh_ff_plan(cgb_op *op) {
         free_ff_plan(op);
         return CGB_OK;
     }
-    return build_images(op, f);
+    CGB_TRY(build_images(op, f));
+    // the next product may be on a stream that the legacy one does not order
+    CGB_CUDA(cudaStreamSynchronize(nullptr));
+    return CGB_OK;
 }
 
 // A x with the table in shared memory; *ran = 0 when the pair kernels are to do it
