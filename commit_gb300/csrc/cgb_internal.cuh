@@ -213,6 +213,8 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
 int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, const double *sqw, const double *ax_a,
                   const double *ax_b, double ca, double cb, double *partials, cudaStream_t st, int *grid,
                   const double **z);
+// after a new table: the plan's images are queued, then (its signs known) completed or the plan is dropped
+int queue_ff_images(cgb_op *op);
 int refresh_ff_plan(cgb_op *op);
 void free_ff_plan(cgb_op *op);
 int ensure_runs(cgb_op *op);

@@ -581,7 +581,8 @@ int cgb_op_set_lut(cgb_op *op, const float *lutIC, const float *lutEC, const flo
     }
     op->lut_r_kind = 0;  // reduced-precision copies are rebuilt on their next use
     op->mixp_kind[0] = op->mixp_kind[1] = 0;
-    CGB_TRY(update_lut_exponents(op));
+    CGB_TRY(queue_ff_images(op));
+    CGB_TRY(update_lut_exponents(op));  // waits for the table and the images
     return refresh_ff_plan(op);
 }
 

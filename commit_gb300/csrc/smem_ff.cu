@@ -98,13 +98,36 @@ __global__ void k_adj_image(const float *__restrict__ lut, int nIC, int ndirs, i
     }
 }
 
-__global__ void k_col_max(const float *__restrict__ lut, int rows, int nS, int padded, float *__restrict__ colmax) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= padded) return;
-    float m = 0.f;
-    if (s < nS)
-        for (int r = 0; r < rows; ++r) m = fmaxf(m, lut[(size_t)r * nS + s]);
-    colmax[s] = m;
+// Column maxima (zero beyond nS; 32 samples per block) and, in the blocks from kColPad / 32 on, the
+// smallest sum of eight rows each; of a non-negative table
+__global__ void __launch_bounds__(256) k_table_bounds(const float *__restrict__ lut, int rows, int nS,
+                                                      float *__restrict__ colmax, float *__restrict__ rowmin) {
+    __shared__ float red[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int rb = (int)blockIdx.x - kColPad / 32;
+    if (rb < 0) {
+        const int s = blockIdx.x * 32 + lane;
+        float m = 0.f;
+        if (s < nS)
+            for (int r = w; r < rows; r += 8) m = fmaxf(m, lut[(size_t)r * nS + s]);
+        red[w][lane] = m;
+        __syncthreads();
+        if (w) return;
+        for (int q = 1; q < 8; ++q) m = fmaxf(m, red[q][lane]);
+        colmax[s] = m;
+    } else {
+        const int r = rb * 8 + w;
+        float t = 0.f;
+        if (r < rows)
+            for (int s = lane; s < nS; s += 32) t += lut[(size_t)r * nS + s];
+#pragma unroll
+        for (int d = 16; d; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+        if (lane == 0) red[w][0] = r < rows ? t : 3.4e38f;
+        __syncthreads();
+        if (threadIdx.x) return;
+        for (int q = 1; q < 8; ++q) t = fminf(t, red[q][0]);
+        rowmin[rb] = t;
+    }
 }
 
 __global__ void k_eval_flags(const uint32_t *__restrict__ eval, int64_t n, unsigned *__restrict__ flags) {
@@ -227,7 +250,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_fwd_smem(const __grid_consta
         for (int i = 0; i < A.nIC; ++i)
             for (uint32_t j = rb + sub; j < re; j += 8) {
                 const float h = A.coef[(size_t)i * A.nruns + j].x;
-                ok = ok && h >= 0.f && h <= 3.0e38f;
+                ok = ok && h >= 0.f && h <= A.coef_max;
                 cm = fmaxf(cm, h);
             }
         __syncwarp();
@@ -498,7 +521,7 @@ __global__ void __launch_bounds__(adj_threads(NP), 1) k_adj_smem(const __grid_co
         const uint32_t rbn = vn >= 0 ? rb_of[vn] : 0u, ren = vn >= 0 ? re_of[vn] : 0u;
         const int vnn = voxel(w + lg + 2 * stride);
         f2 zh[NP], zl[NP];
-        unsigned zmax = 0, neg = 0;
+        unsigned zmax = 0, neg = A.general;
         auto load = [&](int k, double &z0, double &z1) {
             const int s = s_base + 2 * (sub + 8 * kk(k));
             z0 = z1 = 0.0;
@@ -551,10 +574,10 @@ __global__ void __launch_bounds__(adj_threads(NP), 1) k_adj_smem(const __grid_co
         }
         // rows without a negative entry take the five-operation sums (file comment of
         // smem_ff.cuh): the bias is a power of two just below this lane's largest term bound
-        const bool pos = ((__ballot_sync(full, (neg >> 31) != 0u) >> ((threadIdx.x & 31) & ~7)) & 0xffu) == 0u;
-        const bool any_pos = __any_sync(full, pos), any_mix = __any_sync(full, !pos);
-        f2 bias;
-        {
+        bool pos = ((__ballot_sync(full, (neg >> 31) != 0u) >> ((threadIdx.x & 31) & ~7)) & 0xffu) == 0u;
+        f2 bias = 0ull;
+        float low = 0.f;  // smallest dot product that the lanes' biases do not dwarf
+        if (__any_sync(full, pos)) {
             float x0 = 0.f, x1 = 0.f;
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
@@ -564,92 +587,109 @@ __global__ void __launch_bounds__(adj_threads(NP), 1) k_adj_smem(const __grid_co
                 x1 = fmaxf(x1, a1);
             }
             auto down = [](float b) { return __uint_as_float(__float_as_uint(b * 1.001f) & 0x7f800000u); };
-            bias = f2_pack(down(x0), down(x1));
+            x0 = down(x0);
+            x1 = down(x1);
+            bias = f2_pack(x0, x1);
+            low = x0 + x1;
+#pragma unroll
+            for (int d = 4; d; d >>= 1) low += __shfl_xor_sync(full, low, d, 8);
+            low *= 1.f / kBiasAdj;
         }
         int most = (int)(re - rb);
         most = max(most, __shfl_xor_sync(full, most, 8));
         most = max(most, __shfl_xor_sync(full, most, 16));
         if (most == 0) on = rbn + own < ren ? __ldg(A.run_o + rbn + own) : 0u;
-        // Eight runs at a time, four by four: run t of the batch belongs to lane (t & 3) * 2 + (t >> 2),
-        // which is where the butterfly leaves its dot product.
+        // once more with the general sums where the biased ones gave a dot product that the bias dwarfs
 #pragma unroll 1
-        for (int b = 0; b < most; b += 8) {
-            const uint32_t j = rb + b + own;
-            const bool valid = j < re;
-            const unsigned o = valid ? on - (unsigned)(blk * A.no) : 0u;
-            const uint32_t jn = b + 8 < most ? j + 8 : rbn + own;
-            on = jn < (b + 8 < most ? re : ren) ? __ldg(A.run_o + jn) : 0u;
+        for (;;) {
+            const bool any_pos = __any_sync(full, pos), any_mix = __any_sync(full, !pos);
+            bool small = false;
+            // Eight runs at a time, four by four: run t of the batch belongs to lane (t & 3) * 2 + (t >> 2),
+            // which is where the butterfly leaves its dot product.
 #pragma unroll 1
-            for (int i = 0; i < A.nIC; ++i) {
-                const unsigned row = ((unsigned)(i * A.no) + o) * (unsigned)CS;
-                // four dot products' partial sums, of one sign (the bias is a power of two not above
-                // the sums: the difference is exact) or of any
-                auto four_pos = [&](int u) {
-                    DD2 P[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const unsigned r = __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8);
-                        const f2 L0 = pair(r, 0);
-                        const f2 s = f2_fma(zh[0], L0, bias);
-                        P[q].e = f2_fma(zl[0], L0, f2_fma(zh[0], L0, f2_sub(bias, s)));
-                        P[q].s = s;
-#pragma unroll
-                        for (int k = 1; k < NP; ++k) dd2_fma_same(P[q], zh[k], zl[k], pair(r, k));
-                        P[q].s = f2_sub(P[q].s, bias);
-                    }
-                    scatter4(P);
-                    return P[0];
-                };
-                auto four_any = [&](int u) {
-                    DD2 P[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const unsigned r = __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8);
-                        const f2 L0 = pair(r, 0);
-                        const f2 s = f2_fma(zh[0], L0, A.zero);
-                        P[q].e = f2_fma(zl[0], L0, f2_fma(zh[0], L0, f2_neg(s)));
-                        P[q].s = s;
-#pragma unroll
-                        for (int k = 1; k < NP; ++k) dd2_fma_any(P[q], zh[k], zl[k], pair(r, k), A.zero);
-                    }
-                    scatter4(P);
-                    return P[0];
-                };
-                // the lanes of even parity finish the first four, those of odd parity the others
-                DD2 M, N;
-                dd2_zero(M);
+            for (int b = 0; b < most; b += 8) {
+                const uint32_t j = rb + b + own;
+                const bool valid = j < re;
+                const unsigned o = valid ? on - (unsigned)(blk * A.no) : 0u;
+                const uint32_t jn = b + 8 < most ? j + 8 : rbn + own;
+                on = jn < (b + 8 < most ? re : ren) ? __ldg(A.run_o + jn) : 0u;
 #pragma unroll 1
-                for (int u = 0; u < 2; ++u) {
-                    N = M;
-                    if (u && b + 4 >= most) {
-                        dd2_zero(M);
-                        break;
+                for (int i = 0; i < A.nIC; ++i) {
+                    const unsigned row = ((unsigned)(i * A.no) + o) * (unsigned)CS;
+                    // four dot products' partial sums, of one sign (the bias is a power of two not above
+                    // the sums: the difference is exact) or of any
+                    auto four_pos = [&](int u) {
+                        DD2 P[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const unsigned r = __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8);
+                            const f2 L0 = pair(r, 0);
+                            const f2 s = f2_fma(zh[0], L0, bias);
+                            P[q].e = f2_fma(zl[0], L0, f2_fma(zh[0], L0, f2_sub(bias, s)));
+                            P[q].s = s;
+#pragma unroll
+                            for (int k = 1; k < NP; ++k) dd2_fma_same(P[q], zh[k], zl[k], pair(r, k));
+                            P[q].s = f2_sub(P[q].s, bias);
+                        }
+                        scatter4(P);
+                        return P[0];
+                    };
+                    auto four_any = [&](int u) {
+                        DD2 P[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const unsigned r = __shfl_sync(full, row, ((q ^ (sub >> 1)) << 1) + u, 8);
+                            const f2 L0 = pair(r, 0);
+                            const f2 s = f2_fma(zh[0], L0, A.zero);
+                            P[q].e = f2_fma(zl[0], L0, f2_fma(zh[0], L0, f2_neg(s)));
+                            P[q].s = s;
+#pragma unroll
+                            for (int k = 1; k < NP; ++k) dd2_fma_any(P[q], zh[k], zl[k], pair(r, k), A.zero);
+                        }
+                        scatter4(P);
+                        return P[0];
+                    };
+                    // the lanes of even parity finish the first four, those of odd parity the others
+                    DD2 M, N;
+                    dd2_zero(M);
+#pragma unroll 1
+                    for (int u = 0; u < 2; ++u) {
+                        N = M;
+                        if (u && b + 4 >= most) {
+                            dd2_zero(M);
+                            break;
+                        }
+                        if (any_pos) M = four_pos(u);
+                        if (any_mix) {
+                            const DD2 Q = four_any(u);
+                            if (any_pos) M.s = pos ? M.s : Q.s, M.e = pos ? M.e : Q.e;
+                            else M = Q;
+                        }
                     }
-                    if (any_pos) M = four_pos(u);
-                    if (any_mix) {
-                        const DD2 Q = four_any(u);
-                        if (any_pos) M.s = pos ? M.s : Q.s, M.e = pos ? M.e : Q.e;
-                        else M = Q;
+                    const bool odd = (sub & 1) != 0;
+                    DD2 send, keep;
+                    send.s = odd ? N.s : M.s;  // N the first four, M the others
+                    send.e = odd ? N.e : M.e;
+                    keep.s = odd ? M.s : N.s;
+                    keep.e = odd ? M.e : N.e;
+                    dd2_add(keep, dd2_shfl_xor(full, send, 1, 8));
+                    if (valid) {
+                        float ds, de, s1, e1;
+                        f2_unpack(keep.s, ds, s1);
+                        f2_unpack(keep.e, de, e1);
+                        ff_add(ds, de, s1, e1);
+                        small = small || !(ds >= low);
+                        double t = ff_join(ds, de);
+                        if (ez) t = t * pow2(ez);
+                        A.part[((size_t)i * A.nruns + j) * A.nc + chunk] = t;
                     }
+                    __syncwarp();
                 }
-                const bool odd = (sub & 1) != 0;
-                DD2 send, keep;
-                send.s = odd ? N.s : M.s;  // N the first four, M the others
-                send.e = odd ? N.e : M.e;
-                keep.s = odd ? M.s : N.s;
-                keep.e = odd ? M.e : N.e;
-                dd2_add(keep, dd2_shfl_xor(full, send, 1, 8));
-                if (valid) {
-                    float ds, de, s1, e1;
-                    f2_unpack(keep.s, ds, s1);
-                    f2_unpack(keep.e, de, e1);
-                    ff_add(ds, de, s1, e1);
-                    double t = ff_join(ds, de);
-                    if (ez) t = t * pow2(ez);
-                    A.part[((size_t)i * A.nruns + j) * A.nc + chunk] = t;
-                }
-                __syncwarp();
             }
+            const unsigned bad = __ballot_sync(full, pos && small);
+            if (!bad) break;
+            pos = pos && !(bad >> ((threadIdx.x & 31) & ~7) & 0xffu);
+            on = rb + own < re ? __ldg(A.run_o + rb + own) : 0u;
         }
         const unsigned tile = (unsigned)(A.p0 + w) / 4u;
         const bool ends = tile % (unsigned)A.nb == (unsigned)blk;  // this range takes the voxels' EC / ISO elements
@@ -841,7 +881,8 @@ void drop_runs(RunLayout *R) {
     delete R;
 }
 
-int build_images(cgb_op *op, FfPlan *f) {
+// table images, column maxima and row sums, queued on the legacy stream
+int queue_images(cgb_op *op, FfPlan *f) {
     const int rows = op->nIC * op->ndirs;
     if (f->fimg)
         k_fwd_image<<<grid_n((int64_t)f->fnc * rows * f->fcs), 256>>>(op->lutIC, rows, op->nS, f->fnc, 16 * f->fnp,
@@ -849,9 +890,21 @@ int build_images(cgb_op *op, FfPlan *f) {
     if (f->aimg)
         k_adj_image<<<grid_n((int64_t)f->anc * f->anb * op->nIC * f->ano * f->acs), 256>>>(
             op->lutIC, op->nIC, op->ndirs, op->nS, f->anc, 16 * f->anp, f->anb, f->ano, f->acs, f->aimg);
-    const int padded = kMaxSamples + 128;
-    k_col_max<<<(padded + 63) / 64, 64>>>(op->lutIC, rows, op->nS, padded, f->colmax);
+    k_table_bounds<<<kColPad / 32 + (rows + 7) / 8, 256>>>(op->lutIC, rows, op->nS, f->colmax, f->colmax + kColPad);
     CGB_CUDA(cudaGetLastError());
+    return CGB_OK;
+}
+
+// whether the table's rows are uneven; waits for the images (the next product may be on a stream
+// that the legacy one does not order)
+int finish_images(cgb_op *op, FfPlan *f) {
+    const int nb = (op->nIC * op->ndirs + 7) / 8;
+    std::vector<float> b((size_t)kColPad + nb);
+    CGB_CUDA(cudaMemcpy(b.data(), f->colmax, b.size() * sizeof(float), cudaMemcpyDeviceToHost));
+    double sum = 0.0, low = b[kColPad];
+    for (int s = 0; s < op->nS; ++s) sum += b[s];
+    for (int r = 1; r < nb; ++r) low = b[kColPad + r] < low ? b[kColPad + r] : low;
+    f->uneven = !(sum <= kBiasA * low);
     return CGB_OK;
 }
 
@@ -904,7 +957,7 @@ int build_plan(cgb_op *op, FfPlan *f) {
     if ((!fs && !as) || op->lut_signed) return CGB_OK;  // the pair kernels skip zero coefficients, these may multiply by one
     CGB_TRY(ensure_runs(op));
     const RunLayout *R = op->runs;
-    CGB_TRY(keep(op, &f->colmax, (size_t)kMaxSamples + 128));
+    CGB_TRY(keep(op, &f->colmax, (size_t)kColPad + (op->nIC * op->ndirs + 7) / 8));
     if (fs) {
         CGB_TRY(keep(op, &f->fimg, (size_t)f->fnc * op->nIC * op->ndirs * f->fcs));
         CGB_TRY(keep(op, &f->coef, (size_t)op->nIC * R->nruns));
@@ -918,7 +971,8 @@ int build_plan(cgb_op *op, FfPlan *f) {
         CGB_TRY(keep(op, &f->run_blk, (size_t)(f->anb + 1) * nV));
         k_run_blk<<<(nV + 255) / 256, 256>>>(R->run_ptr, R->run_o, nV, f->anb, f->ano, f->run_blk);
     }
-    CGB_TRY(build_images(op, f));
+    CGB_TRY(queue_images(op, f));
+    CGB_TRY(finish_images(op, f));
     CGB_CUDA(cudaDeviceSynchronize());
     f->fwd_ok = fs;
     f->adj_ok = as;
@@ -1030,6 +1084,8 @@ static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
     return CGB_OK;
 }
 
+int queue_ff_images(cgb_op *op) { return op->ffp && op->ffp->colmax ? queue_images(op, op->ffp) : CGB_OK; }
+
 int refresh_ff_plan(cgb_op *op) {
     if (!op->ffp) return CGB_OK;
     FfPlan *f = op->ffp;
@@ -1037,10 +1093,7 @@ int refresh_ff_plan(cgb_op *op) {
         free_ff_plan(op);
         return CGB_OK;
     }
-    CGB_TRY(build_images(op, f));
-    // the next product may be on a stream that the legacy one does not order
-    CGB_CUDA(cudaStreamSynchronize(nullptr));
-    return CGB_OK;
+    return finish_images(op, f);
 }
 
 // A x with the table in shared memory; *ran = 0 when the pair kernels are to do it
@@ -1056,6 +1109,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     const RunLayout &R = *op->runs;
     a.vperm = R.vperm; a.run_ptr = R.run_ptr; a.run_o = R.run_o; a.coef = f->coef; a.nruns = R.nruns;
     a.img = f->fimg; a.colmax = f->colmax;
+    a.coef_max = f->uneven ? -1.f : 3.0e38f;
     a.nIC = op->nIC; a.ndirs = op->ndirs; a.nS = op->nS; a.nc = f->fnc;
     perm_range(op, a.v0, a.v1, a.p0, a.p1);
     a.ec_ptr = op->ec_ptr; a.ec_col = op->ec_col; a.ec_o = op->ec_o; a.iso_ptr = op->iso_ptr; a.iso_col = op->iso_col;
@@ -1107,6 +1161,7 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
     const RunLayout &R = *op->runs;
     a.vperm = R.vperm; a.run_blk = f->run_blk; a.run_seg = R.run_seg; a.run_o = R.run_o; a.seg_l = op->seg_l;
     a.n = op->n; a.nruns = R.nruns; a.img = f->aimg; a.colmax = f->colmax;
+    a.general = f->uneven ? 0x80000000u : 0u;
     a.nIC = op->nIC; a.nS = op->nS; a.nV = op->nV; a.nc = f->anc; a.nb = f->anb; a.no = f->ano;
     perm_range(op, a.v0, a.v1, a.p0, a.p1);
     a.ec_ptr = op->ec_ptr; a.ec_col = op->ec_col; a.ec_o = op->ec_o; a.iso_ptr = op->iso_ptr; a.iso_col = op->iso_col;

@@ -21,8 +21,19 @@
 //   A   x >= 0 and table >= 0 (checked per voxel / per handle): the first 8 runs are added
 //       with the general two-sum, the bias tops s up to max(c) * max(column) where it is
 //       below, and s, e are renormalised every 8 terms;
-//   A'  the bias is the sum of the negative terms' bounds plus the largest one, per lane.
-// Voxels with a negative or non-finite coefficient use the general two-sum throughout.
+//   A'  row and table >= 0: the bias is the power of two just below the lane's largest term bound,
+//       so that the sums neither cancel nor let the bias take their last bits.
+// Voxels with a negative or non-finite coefficient and rows with a negative entry use the general
+// two-sum throughout.
+// The error is relative to sum + bias, and the bias follows the largest table value of each sample,
+// whether the voxel has that row or not.  So it may be at most kBiasA times a voxel's own sum (A: a
+// rule on the table, FfPlan::uneven, since the sum is at least the largest coefficient times the
+// smallest row) and kBiasAdj times a dot product (A': the same rule, and every dot product is looked
+// at), else the general sums are taken.  120 runs a voxel and an unused row 10^6 times as large: A was
+// off by 2e-9 of a voxel's norm with the bias.  Rows that are rotations of one response have column
+// maxima of 1.6 (b = 1000) to 3.8 (b = 10000 s/mm^2) times a row and biases up to 1.5 times a dot
+// product for measured signals.  Cost, us a pair: 288 samples, 122 M segments 20580 / 20580,
+// 15 M 4870 / 4850, three responses x 99 samples 901 / 908.
 #pragma once
 #include "operator_pair.cuh"
 
@@ -45,7 +56,9 @@ struct FfPlan {
     // A: samples in fnc chunks of 16 * fnp, row stride fcs floats
     int fnp, fnc, fcs;
     float *fimg;                 // [fnc][nIC * ndirs][fcs]
-    float *colmax;               // [>= nS] largest table value per sample, zero beyond nS
+    float *colmax;               // [kColPad] largest table value per sample, zero beyond nS; then
+                                 // the smallest row sum of every eight rows
+    int uneven;                  // sum(colmax) > kBiasA * the smallest row sum: no biased sums
     // A': samples in anc chunks of 16 * anp, orientations in anb ranges of ano, row stride acs
     int anp, anc, anb, ano, acs;
     float *aimg;                 // [anc][anb][nIC * ano][acs]
@@ -59,6 +72,8 @@ struct FfPlan {
 };
 
 constexpr int kVoxWindow = 4096;
+constexpr int kColPad = kMaxSamples + 128;
+constexpr float kBiasA = 4.f, kBiasAdj = 8.f;  // largest bias against the sums it joins (file comment)
 // threads of the one block per SM: 80 registers a thread, and 96 where A' needs them (measured at 5
 // and 6 pairs per lane: 45 and 1900 us with 640 threads, 49 and 1940 with 768; at 4: 616 and 571)
 constexpr int kFwdThreads = 768;
@@ -137,6 +152,7 @@ struct SmFwdArgs {
     const float2 *coef;
     int64_t nruns;
     const float *img, *colmax;
+    float coef_max;                           // largest coefficient of the fast sums (uneven table: none)
     int nIC, ndirs, nS, nc, p0, p1, v0, v1;   // perm positions [p0, p1), voxels [v0, v1)
     const uint32_t *ec_ptr, *ec_col, *iso_ptr, *iso_col;
     const uint16_t *ec_o;
@@ -159,6 +175,7 @@ struct SmAdjArgs {
     const float *seg_l;
     int64_t n, nruns;
     const float *img, *colmax;
+    unsigned general;                         // sign bit: general sums for every row (uneven table)
     int nIC, nS, nV, nc, nb, no, p0, p1, v0, v1;
     const uint32_t *ec_ptr, *ec_col, *iso_ptr, *iso_col;
     const uint16_t *ec_o;
