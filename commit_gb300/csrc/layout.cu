@@ -32,6 +32,7 @@ int fail(int code, const std::string &msg) {
 }
 
 int cuda_fail(cudaError_t e, const char *what) {
+    cudaGetLastError();  // the launch checks of the next call are not to find this call's error
     g_last_error = std::string("CUDA error in ") + what + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? CGB_ERR_NOMEM : CGB_ERR_CUDA;
 }

@@ -20,6 +20,7 @@
 // 2.9 M runs x 66 multiply-adds are 0.44 ms of that pipe.
 #include <cub/cub.cuh>
 
+#include <memory>
 #include <vector>
 
 #include "cgb_internal.cuh"
@@ -319,8 +320,7 @@ struct LutGradState {
 
 static int ensure_grad_state(cgb_op *op) {
     if (op->gstate) return CGB_OK;
-    LutGradState *G = new LutGradState();
-    op->gstate = G;
+    std::unique_ptr<LutGradState> G(new LutGradState());
     if (op->nIC > 0 && op->n > 0)
         CGB_TRY(build_stream(op->seg_o, op->vox_ptr, op->nV, op->n, op->ndirs, op->nsm, G->ic));
     if (op->nEC > 0 && op->nE > 0)
@@ -330,6 +330,7 @@ static int ensure_grad_state(cgb_op *op) {
     CGB_CUDA(cudaMalloc((void **)&G->partial, (need ? need : 1) * sizeof(double)));
     G->partial_len = need;
     CGB_CUDA(cudaDeviceSynchronize());
+    op->gstate = G.release();  // complete: a call that failed on the way leaves none
     return CGB_OK;
 }
 
