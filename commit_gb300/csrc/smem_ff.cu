@@ -951,10 +951,15 @@ int build_runs(cgb_op *op, RunLayout *R) {
     return CGB_OK;
 }
 
+bool dense(const cgb_op *op, double items) { return (double)op->n * op->nIC >= items * op->nV; }
+
+// the directions whose shape and density suit these kernels, and nothing for the others
 int build_plan(cgb_op *op, FfPlan *f) {
     const int nV = op->nV;
-    const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f), as = adj_shape(op->nIC, op->ndirs, op->nS, f);
-    if ((!fs && !as) || op->lut_signed) return CGB_OK;  // the pair kernels skip zero coefficients, these may multiply by one
+    if (op->lut_signed) return CGB_OK;  // the pair kernels skip zero coefficients, these may multiply by one
+    const bool fs = fwd_shape(op->nIC * op->ndirs, op->nS, f) && dense(op, smem_min_items(op->nS, f->fnc));
+    const bool as = adj_shape(op->nIC, op->ndirs, op->nS, f) && dense(op, smem_min_items(op->nS, f->anc * f->anb));
+    if (!fs && !as) return CGB_OK;
     CGB_TRY(ensure_runs(op));
     const RunLayout *R = op->runs;
     CGB_TRY(keep(op, &f->colmax, (size_t)kColPad + (op->nIC * op->ndirs + 7) / 8));
@@ -978,8 +983,6 @@ int build_plan(cgb_op *op, FfPlan *f) {
     f->adj_ok = as;
     return CGB_OK;
 }
-
-bool dense(const cgb_op *op, double items) { return (double)op->n * op->nIC >= items * op->nV; }
 
 bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1102,7 +1105,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     *ran = 0;
     FfPlan *f;
     CGB_TRY(plan_for(op, st, &f));
-    if (!f || !f->fwd_ok || !dense(op, smem_min_items(op->nS, f->fnc))) return CGB_OK;
+    if (!f || !f->fwd_ok) return CGB_OK;
     const OpDev P = op->dev();
     SmFwdArgs a;
     memset(&a, 0, sizeof(a));
@@ -1154,7 +1157,7 @@ int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int
     *ran = 0;
     FfPlan *f;
     CGB_TRY(plan_for(op, st, &f));
-    if (!f || !f->adj_ok || !dense(op, smem_min_items(op->nS, f->anc * f->anb))) return CGB_OK;
+    if (!f || !f->adj_ok) return CGB_OK;
     const OpDev P = op->dev();
     SmAdjArgs a;
     memset(&a, 0, sizeof(a));
@@ -1199,7 +1202,7 @@ int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, 
     *z = nullptr;
     FfPlan *f;
     CGB_TRY(plan_for(op, st, &f));
-    if (!f || !f->adj_ok || !f->fwd_ok || !dense(op, smem_min_items(op->nS, f->anc * f->anb))) return CGB_OK;
+    if (!f || !f->adj_ok || !f->fwd_ok) return CGB_OK;
     if (!f->zrow) {
         if (capturing(st)) return CGB_OK;
         const int rc = keep(op, &f->zrow, (size_t)op->nrows);

@@ -1,0 +1,48 @@
+"""Which products take the kernels that keep the table in shared memory, and what the handle holds for them."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import golden_io as G
+import oracle as O
+from kernel_trace import ran
+from test_smem_products_gpu import TOL, _problem
+
+pytestmark = pytest.mark.gpu
+
+
+# segments x responses per voxel below and above 4 per chunk of 96 samples (two chunks: 8), far below
+# for three chunks (12), and between A' (two orientation ranges: 12) and A (three chunks for one: 20)
+@pytest.mark.parametrize('nS,n_fibers,nIC,ndirs,fwd,adj', [
+    (97, 3000, 1, 120, False, False), (97, 3800, 1, 120, True, True), (288, 2500, 1, 120, False, False),
+    (70, 3000, 2, 500, False, True), (70, 5000, 2, 500, True, True)])
+def test_layout_only_for_the_products_that_use_it(nS, n_fibers, nIC, ndirs, fwd, adj):
+    """An operator too sparse for these kernels holds nothing for them; one dense enough for A' only
+    holds no run coefficients."""
+    from commit_gb300.operator import LinearOperator
+    D, K = _problem(nS, n_fibers, n_mask=60000, dim=(60, 60, 40), ndirs=ndirs, nIC=nIC)
+    IC = D['IC']
+    per = IC['n'] * nIC / IC['nVOX']
+    chunks = -(-nS // 96)
+    low_a, low_at = (20.0, 12.0) if nIC == 2 else (4.0 * chunks,) * 2
+    assert IC['n'] * nIC * nS >= 1e7 and (per >= low_a) == fwd and (per >= low_at) == adj
+    A, P = LinearOperator(D, K, None), O.PortOperator(D, K, None, nthreads=8)
+    rng = np.random.default_rng(0)
+    x, y = rng.uniform(0, 1, A.nCOLS), rng.normal(size=A.nROWS)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    before = A.device_bytes()
+    assert G.rel(A.dot(xd).cpu().numpy(), P.dot(x)) <= TOL
+    assert G.rel(A.T.dot(yd).cpu().numpy(), P.T.dot(y)) <= TOL
+    held = A.device_bytes() - before
+    v, runs = IC['nVOX'], np.unique(IC['vox'].astype(np.int64) * ndirs + IC['dir']).size
+    layout, coef, part = 8 * v + 6 * runs, 8 * nIC * runs, 8 * nIC * runs * chunks
+    want = (layout + part + (coef if fwd else 0)) if adj else 0
+    small = (2 << 20) + 4 * 4 * v                                # table images, orientation ranges, EC / ISO parts
+    if chunks > 1:
+        small += 8 * chunks * (D['EC']['n'] + 2 * D['ISO']['n'])
+    assert want <= held <= want + (small if want else 0)
+    assert fwd == adj or small < coef                            # the bound tells the coefficients apart
+    assert ran(lambda: A.dot(xd), 'k_fwd_smem', 'k_forward_p') == [fwd, not fwd]
+    assert ran(lambda: A.T.dot(yd), 'k_adj_smem', 'k_adjoint_p') == [adj, not adj]
