@@ -828,13 +828,6 @@ struct Buf {
     }
 };
 
-template <class T>
-int keep(cgb_op *op, T **p, size_t count) {
-    CGB_CUDA(cudaMalloc((void **)p, (count ? count : 1) * sizeof(T)));
-    op->bytes += (count ? count : 1) * sizeof(T);
-    return CGB_OK;
-}
-
 constexpr size_t kTableBytes = 224 << 10;  // of the 227 KB a block may have
 
 // sample chunks of A: the fewest whose table part fits, at most 6 pairs per lane
@@ -874,10 +867,11 @@ bool adj_shape(int nIC, int ndirs, int nS, FfPlan *f) {
     return best <= 16;
 }
 
-void drop_runs(RunLayout *R) {
+void drop_runs(cgb_op *op, RunLayout *R) {
     void *p[] = {R->run_ptr, R->run_o, R->run_seg, R->vperm};
     for (void *q : p)
         if (q) cudaFree(q);
+    op->bytes -= R->bytes;
     delete R;
 }
 
@@ -939,10 +933,10 @@ int build_runs(cgb_op *op, RunLayout *R) {
     CGB_CUDA(cudaMemcpy(&hf, flags, 4, cudaMemcpyDeviceToHost));
     R->nruns = (int64_t)lastid[0] + lastid[1];
     R->eval_ones = hf == 0u;
-    CGB_TRY(keep(op, &R->run_ptr, (size_t)nV + 1));
-    CGB_TRY(keep(op, &R->run_o, (size_t)R->nruns));
-    CGB_TRY(keep(op, &R->run_seg, (size_t)R->nruns + 1));
-    CGB_TRY(keep(op, &R->vperm, (size_t)nV));
+    CGB_TRY(keep_buffer(op, &R->bytes, &R->run_ptr, (size_t)nV + 1));
+    CGB_TRY(keep_buffer(op, &R->bytes, &R->run_o, (size_t)R->nruns));
+    CGB_TRY(keep_buffer(op, &R->bytes, &R->run_seg, (size_t)R->nruns + 1));
+    CGB_TRY(keep_buffer(op, &R->bytes, &R->vperm, (size_t)nV));
     k_run_fill<<<grid_n(n), 256>>>(head, id, op->seg_o, n, (uint32_t)R->nruns, R->run_o, R->run_seg);
     k_run_ptr<<<(nV + 256) / 256, 256>>>(op->vox_ptr, id, nV, n, (uint32_t)R->nruns, R->run_ptr);
     k_perm_key<<<(nV + 255) / 256, 256>>>(R->run_ptr, nV, key, val);
@@ -962,18 +956,18 @@ int build_plan(cgb_op *op, FfPlan *f) {
     if (!fs && !as) return CGB_OK;
     CGB_TRY(ensure_runs(op));
     const RunLayout *R = op->runs;
-    CGB_TRY(keep(op, &f->colmax, (size_t)kColPad + (op->nIC * op->ndirs + 7) / 8));
+    CGB_TRY(keep_buffer(op, &f->bytes, &f->colmax, (size_t)kColPad + (op->nIC * op->ndirs + 7) / 8));
     if (fs) {
-        CGB_TRY(keep(op, &f->fimg, (size_t)f->fnc * op->nIC * op->ndirs * f->fcs));
-        CGB_TRY(keep(op, &f->coef, (size_t)op->nIC * R->nruns));
+        CGB_TRY(keep_buffer(op, &f->bytes, &f->fimg, (size_t)f->fnc * op->nIC * op->ndirs * f->fcs));
+        CGB_TRY(keep_buffer(op, &f->bytes, &f->coef, (size_t)op->nIC * R->nruns));
         CGB_CUDA(cudaEventCreateWithFlags(&f->done, cudaEventDisableTiming));
     }
     if (as) {
-        CGB_TRY(keep(op, &f->aimg, (size_t)f->anc * f->anb * op->nIC * f->ano * f->acs));
-        CGB_TRY(keep(op, &f->part, (size_t)op->nIC * R->nruns * f->anc));
+        CGB_TRY(keep_buffer(op, &f->bytes, &f->aimg, (size_t)f->anc * f->anb * op->nIC * f->ano * f->acs));
+        CGB_TRY(keep_buffer(op, &f->bytes, &f->part, (size_t)op->nIC * R->nruns * f->anc));
         if (f->anc > 1)
-            CGB_TRY(keep(op, &f->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * f->anc));
-        CGB_TRY(keep(op, &f->run_blk, (size_t)(f->anb + 1) * nV));
+            CGB_TRY(keep_buffer(op, &f->bytes, &f->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * f->anc));
+        CGB_TRY(keep_buffer(op, &f->bytes, &f->run_blk, (size_t)(f->anb + 1) * nV));
         k_run_blk<<<(nV + 255) / 256, 256>>>(R->run_ptr, R->run_o, nV, f->anb, f->ano, f->run_blk);
     }
     CGB_TRY(queue_images(op, f));
@@ -1030,7 +1024,7 @@ int ensure_runs(cgb_op *op) {
     memset((void *)R, 0, sizeof(RunLayout));
     const int rc = build_runs(op, R);
     if (rc != CGB_OK) {
-        drop_runs(R);
+        drop_runs(op, R);
         return rc;
     }
     op->runs = R;
@@ -1038,21 +1032,22 @@ int ensure_runs(cgb_op *op) {
 }
 
 void free_runs(cgb_op *op) {
-    if (op->runs) drop_runs(op->runs);
+    if (op->runs) drop_runs(op, op->runs);
     op->runs = nullptr;
 }
 
-static void drop_plan(FfPlan *f) {
+static void drop_plan(cgb_op *op, FfPlan *f) {
     void *p[] = {f->coef, f->fimg, f->colmax, f->aimg, f->run_blk, f->part, f->epart, f->zrow};
     for (void *q : p)
         if (q) cudaFree(q);
     if (f->done) cudaEventDestroy(f->done);
+    op->bytes -= f->bytes;
     memset((void *)f, 0, sizeof(*f));
 }
 
 void free_ff_plan(cgb_op *op) {
     if (!op->ffp) return;
-    drop_plan(op->ffp);
+    drop_plan(op, op->ffp);
     delete op->ffp;
     op->ffp = nullptr;
 }
@@ -1069,16 +1064,16 @@ static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
         if (!op->ffp) {
             FfPlan *f = new FfPlan();
             memset((void *)f, 0, sizeof(*f));
-            const size_t bytes = op->bytes;
+            const bool had_runs = op->runs != nullptr;
             const int rc = build_plan(op, f);
             if (rc != CGB_OK) {
-                drop_plan(f);
-                op->bytes = bytes;
+                drop_plan(op, f);
+                if (!had_runs) free_runs(op);
                 if (rc != CGB_ERR_NOMEM) {
                     delete f;
                     return rc;
                 }
-                cudaGetLastError();  // no room for the plan: it stays empty and the pair kernels run
+                f->no_room = 1;  // the plan stays empty and the pair kernels run
             }
             op->ffp = f;
         }
@@ -1092,6 +1087,7 @@ int queue_ff_images(cgb_op *op) { return op->ffp && op->ffp->colmax ? queue_imag
 int refresh_ff_plan(cgb_op *op) {
     if (!op->ffp) return CGB_OK;
     FfPlan *f = op->ffp;
+    if (f->no_room) return CGB_OK;
     if (op->lut_signed || !f->colmax) {  // the choice of kernels changed: laid out anew
         free_ff_plan(op);
         return CGB_OK;
@@ -1205,12 +1201,8 @@ int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, 
     if (!f || !f->adj_ok || !f->fwd_ok) return CGB_OK;
     if (!f->zrow) {
         if (capturing(st)) return CGB_OK;
-        const int rc = keep(op, &f->zrow, (size_t)op->nrows);
-        if (rc == CGB_ERR_NOMEM) {
-            cudaGetLastError();
-            f->zrow = nullptr;
-            return CGB_OK;
-        }
+        const int rc = keep_buffer(op, &f->bytes, &f->zrow, (size_t)op->nrows);
+        if (rc == CGB_ERR_NOMEM) return CGB_OK;
         CGB_TRY(rc);
     }
     if (in_mode == 1) {

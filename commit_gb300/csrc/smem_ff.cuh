@@ -47,6 +47,7 @@ struct RunLayout {
     uint32_t *run_seg;           // [nruns+1] first segment
     uint32_t *vperm;             // [nV] voxels, by falling run count within windows of kVoxWindow
     int eval_ones;               // eval is 1 everywhere
+    size_t bytes;                // of the handle's, held here
 };
 
 // Table images and buffers of the shared-memory float-float products
@@ -69,6 +70,8 @@ struct FfPlan {
     cudaEvent_t done;            // the last product that used coef has finished
     cudaStream_t last;           // ... and its stream
     int used;
+    int no_room;                 // the buffers did not fit: not tried again
+    size_t bytes;                // of the handle's, held here
 };
 
 constexpr int kVoxWindow = 4096;
@@ -92,6 +95,16 @@ constexpr double kSmemMinWork = 1e7;
 inline double smem_min_items(int nS, int parts) {
     const int chunks = (nS + 95) / 96;
     return 4.0 * chunks + 8.0 * (parts - chunks);
+}
+
+// device buffers that the handle keeps, counted in its bytes and in `held`
+template <class T>
+int keep_buffer(cgb_op *op, size_t *held, T **p, size_t count) {
+    const size_t b = (count ? count : 1) * sizeof(T);
+    CGB_CUDA(cudaMalloc((void **)p, b));
+    op->bytes += b;
+    *held += b;
+    return CGB_OK;
 }
 
 namespace detail {

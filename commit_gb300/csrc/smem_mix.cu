@@ -121,29 +121,24 @@ bool mix_shape(const cgb_op *op, int word, MixPlan *m) {
     return false;
 }
 
-void drop(MixPlan *m) {
+void drop(cgb_op *op, MixPlan *m) {
     void *p[] = {m->img, m->coef, m->part, m->epart};
     for (void *q : p)
         if (q) cudaFree(q);
+    op->bytes -= m->bytes;
+    m->bytes = 0;
     m->img = nullptr;
     m->coef = m->part = nullptr;
     m->epart = nullptr;
 }
 
-template <class T>
-int take(cgb_op *op, T **p, size_t count) {
-    CGB_CUDA(cudaMalloc((void **)p, (count ? count : 1) * sizeof(T)));
-    op->bytes += (count ? count : 1) * sizeof(T);
-    return CGB_OK;
-}
-
 int build_mix(cgb_op *op, int word, MixPlan *m) {
     CGB_TRY(ensure_runs(op));
     const int64_t runs = op->runs->nruns * op->nIC;
-    CGB_TRY(take(op, &m->coef, (size_t)runs));
-    if (m->nc > 1) CGB_TRY(take(op, &m->part, (size_t)runs * m->nc));
-    if (m->nc > 1) CGB_TRY(take(op, &m->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * m->nc));
-    CGB_TRY(take(op, &m->img, (size_t)m->nc * op->nIC * op->ndirs * m->cs * word));
+    CGB_TRY(keep_buffer(op, &m->bytes, &m->coef, (size_t)runs));
+    if (m->nc > 1) CGB_TRY(keep_buffer(op, &m->bytes, &m->part, (size_t)runs * m->nc));
+    if (m->nc > 1) CGB_TRY(keep_buffer(op, &m->bytes, &m->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * m->nc));
+    CGB_TRY(keep_buffer(op, &m->bytes, &m->img, (size_t)m->nc * op->nIC * op->ndirs * m->cs * word));
     CGB_CUDA(cudaEventCreateWithFlags(&m->done, cudaEventDisableTiming));
     return CGB_OK;
 }
@@ -184,16 +179,16 @@ int mix_plan(cgb_op *op, cudaStream_t st, int arith, int adjoint, MixPlan **out)
         CGB_CUDA(cudaDeviceSynchronize());
         if (!op->mixp[f32]) {
             MixPlan *m = new MixPlan(shape);
-            const size_t bytes = op->bytes;
+            const bool had_runs = op->runs != nullptr;
             const int rc = build_mix(op, word, m);
             if (rc != CGB_OK) {
-                drop(m);
-                op->bytes = bytes;
+                drop(op, m);
+                if (!had_runs) free_runs(op);
                 if (rc != CGB_ERR_NOMEM) {
                     delete m;
                     return rc;
                 }
-                cudaGetLastError();  // no room: the plan stays empty and the gathering kernels run
+                // no room: the plan stays empty and the gathering kernels run
             }
             op->mixp[f32] = m;
         }
@@ -265,7 +260,7 @@ int leave(MixPlan *m, cudaStream_t st) {
 void free_mix_plan(cgb_op *op) {
     for (MixPlan *&m : op->mixp) {
         if (!m) continue;
-        drop(m);
+        drop(op, m);
         if (m->done) cudaEventDestroy(m->done);
         delete m;
         m = nullptr;

@@ -27,6 +27,7 @@ struct MixPlan {
     cudaEvent_t done;    // the last product has finished with the buffers
     cudaStream_t last;   // ... and its stream
     int used;
+    size_t bytes;        // of the handle's, held here
 };
 
 constexpr int kMixThreads = 768;

@@ -1,4 +1,5 @@
-"""Which products take the kernels that keep the table in shared memory, and what the handle holds for them."""
+"""Which products take the kernels that keep the table in shared memory, and what the handle holds
+for them."""
 import ctypes
 
 import numpy as np
@@ -46,3 +47,31 @@ def test_layout_only_for_the_products_that_use_it(nS, n_fibers, nIC, ndirs, fwd,
     assert fwd == adj or small < coef                            # the bound tells the coefficients apart
     assert ran(lambda: A.dot(xd), 'k_fwd_smem', 'k_forward_p') == [fwd, not fwd]
     assert ran(lambda: A.T.dot(yd), 'k_adj_smem', 'k_adjoint_p') == [adj, not adj]
+
+
+def _set_table(A, K):
+    from commit_gb300._lib import check, lib
+    check(lib().cgb_op_set_lut(A.handle, K['wmr'].ctypes.data_as(ctypes.c_void_p), None, None))
+
+
+def test_bytes_follow_the_layout():
+    """A table with a negative entry releases the layout of the FP64 products and the next one builds it again:
+    the handle's bytes do not grow with the changes."""
+    from commit_gb300.operator import LinearOperator
+    D, K = _problem(97, 6000)
+    A = LinearOperator(D, K, None)
+    x, y = torch.rand(A.nCOLS, dtype=torch.float64, device='cuda'), torch.rand(A.nROWS, dtype=torch.float64, device='cuda')
+    neg = dict(K, wmr=K['wmr'].copy())
+    neg['wmr'][0, 0, 0] *= -1
+    start = A.device_bytes()
+    A.dot(x), A.T.dot(y)
+    full = A.device_bytes()
+    for _ in range(3):
+        _set_table(A, neg)
+        A.dot(x), A.T.dot(y)
+        assert start < A.device_bytes() < full
+        _set_table(A, K)
+        A.dot(x), A.T.dot(y)
+        assert A.device_bytes() == full
+    A.dot(x.float(), arith='f32'), A.T.dot(y.float(), arith='f32')
+    assert A.device_bytes() > full
