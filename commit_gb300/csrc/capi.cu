@@ -206,7 +206,7 @@ extern "C" int cgb_op_occupancy(cgb_op *op, int slot, int set, int *choice, floa
     if (set >= 0) {
         if (set > 2) return fail(CGB_ERR_INVALID, "choice must be 0 (retune), 1 or 2");
         op->occ_choice[slot] = set;
-        op->ff_pinned = 1;  // the builds are those of the pair kernels
+        op->occ_set |= 1u << slot;  // the builds are those of the gathering kernels
     }
     if (choice) *choice = op->occ_choice[slot];
     if (ms_a) *ms_a = op->occ_ms[slot][0];

@@ -175,7 +175,8 @@ struct cgb_op {
     cgb::MixPlan *mixp[2];          // buffers of the FP32-vector products (16-bit, FP32 table), likewise
     int mixp_kind[2];               // arithmetic of their table images (0: to be filled)
     cgb::FfPlan *ffp;               // run layout of the shared-memory products, built on first use
-    int ff_pinned;                  // a build or shape of the pair kernels was set: they run
+    int ff_pinned;                  // a shape of the pair kernels was set: no shared-memory products
+    unsigned occ_set;               // slots whose build was set: the products of their kernels run on them
     size_t bytes;
     int nsm;
     cgb::OpDev dev() const;
@@ -355,6 +356,14 @@ enum OccSlot {
     kOccAdjFFWideFused = 18,
     kOccSlots = 24
 };
+
+// the slots of a product's gathering kernels: while one is set (occ_set), the product runs on them
+constexpr unsigned kOccOfFwdFF = 1u << kOccFwdFF | 1u << kOccFwdFFWide;
+constexpr unsigned kOccOfAdjFF = 1u << kOccAdjFF | 1u << kOccAdjFFWide;
+constexpr unsigned kOccOfGradFF = kOccOfFwdFF | kOccOfAdjFF | 1u << kOccAdjFFFused | 1u << kOccAdjFFWideFused;
+constexpr unsigned occ_of_mix(int arith, int adjoint) {
+    return 1u << ((adjoint ? kOccAdjMix : kOccFwdMix) + arith - CGB_ARITH_BF16);
+}
 
 template <class FA, class FB>
 int occ_launch(cgb_op *op, int slot, cudaStream_t st, FA &&a, FB &&b) {

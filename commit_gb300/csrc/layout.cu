@@ -603,6 +603,7 @@ int cgb_op_ff_kernels(cgb_op *op, int variant, int *out) {
     if (!op) return fail(CGB_ERR_INVALID, "null handle");
     if (variant > 1) return fail(CGB_ERR_INVALID, "variant must be 0 (scalar samples) or 1 (packed pairs)");
     if (variant >= 0) op->ff_variant = variant;
+    if (variant == 1) op->ff_pinned = 0, op->occ_set = 0;
     if (out) *out = op->ff_variant;
     return CGB_OK;
 }

@@ -1052,10 +1052,12 @@ void free_ff_plan(cgb_op *op) {
     op->ffp = nullptr;
 }
 
-// the handle's plan if the shared-memory kernels are to run this product, else null
-static int plan_for(cgb_op *op, cudaStream_t st, FfPlan **out) {
+// the handle's plan if the shared-memory kernels are to run this product, else null; `slots`: the pair
+// kernels that would run it otherwise
+static int plan_for(cgb_op *op, cudaStream_t st, unsigned slots, FfPlan **out) {
     *out = nullptr;
-    if (in_place_only() || op->ff_variant != 1 || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
+    if (in_place_only() || op->ff_variant != 1 || op->ff_pinned || (op->occ_set & slots)) return CGB_OK;
+    if (op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
     if (op->nS < 17 || (double)op->n * op->nIC * op->nS < kSmemMinWork) return CGB_OK;
     if (!op->ffp) {
         if (capturing(st)) return CGB_OK;
@@ -1100,7 +1102,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
                  double *partials, cudaStream_t st, int *grid, int *ran) {
     *ran = 0;
     FfPlan *f;
-    CGB_TRY(plan_for(op, st, &f));
+    CGB_TRY(plan_for(op, st, kOccOfFwdFF, &f));
     if (!f || !f->fwd_ok) return CGB_OK;
     const OpDev P = op->dev();
     SmFwdArgs a;
@@ -1152,7 +1154,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
 int adjoint_smem(cgb_op *op, const double *z, double *xout, cudaStream_t st, int *ran) {
     *ran = 0;
     FfPlan *f;
-    CGB_TRY(plan_for(op, st, &f));
+    CGB_TRY(plan_for(op, st, kOccOfAdjFF, &f));
     if (!f || !f->adj_ok) return CGB_OK;
     const OpDev P = op->dev();
     SmAdjArgs a;
@@ -1197,7 +1199,7 @@ int residual_smem(cgb_op *op, int in_mode, const double *x, const double *yobs, 
                   const double **z) {
     *z = nullptr;
     FfPlan *f;
-    CGB_TRY(plan_for(op, st, &f));
+    CGB_TRY(plan_for(op, st, kOccOfGradFF, &f));
     if (!f || !f->adj_ok || !f->fwd_ok) return CGB_OK;
     if (!f->zrow) {
         if (capturing(st)) return CGB_OK;

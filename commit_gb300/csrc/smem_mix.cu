@@ -163,7 +163,8 @@ constexpr int64_t kTcAdjDense = 300;
 // Its buffers stay where they are for the handle's life: the shape does not depend on `arith`.
 int mix_plan(cgb_op *op, cudaStream_t st, int arith, int adjoint, MixPlan **out) {
     *out = nullptr;
-    if (in_place_only() || op->ff_pinned || op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
+    if (in_place_only() || op->ff_pinned || (op->occ_set & occ_of_mix(arith, adjoint))) return CGB_OK;
+    if (op->nolut || op->nIC == 0 || op->n == 0 || op->nF == 0) return CGB_OK;
     const int f32 = arith == CGB_ARITH_F32, word = f32 ? 4 : 2;
     const bool tc = arith == CGB_ARITH_BF16 && tc_forward_enabled(op);
     if (tc && op->tc_mode == 2) return CGB_OK;

@@ -196,7 +196,8 @@ class LinearOperator:
 
     def occupancy(self, set_to: dict | None = None) -> dict:
         """Occupancy autotuning state per tuned kernel: {name: (choice, ms_build1, ms_build2)}
-        (choice 0 = not tuned yet).  ``set_to`` {name: 0|1|2} fixes (or resets) choices."""
+        (choice 0 = not tuned yet).  ``set_to`` {name: 0|1|2} fixes (or resets) choices, and keeps
+        the products of those kernels from the shared-memory ones until ``ff_kernels(1)``."""
         out = {}
         for name, slot in self.OCC_SLOTS.items():
             c, a, b = ctypes.c_int32(), ctypes.c_float(), ctypes.c_float()
@@ -207,15 +208,16 @@ class LinearOperator:
 
     def ff_shape(self, set_to: int | None = None) -> tuple:
         """Voxel shape of the float-float pair kernels (A, A'): 1 default, 2 a warp per voxel,
-        0 timed on the next call; ``set_to`` sets both."""
+        0 timed on the next call; ``set_to`` sets both, and keeps all products from the
+        shared-memory kernels until ``ff_kernels(1)``."""
         f, a = ctypes.c_int32(), ctypes.c_int32()
         check(lib().cgb_op_ff_shape(self._h.ptr, -1 if set_to is None else int(set_to), ctypes.byref(f),
                                     ctypes.byref(a)))
         return int(f.value), int(a.value)
 
     def ff_kernels(self, variant: int | None = None) -> int:
-        """Float-float kernel family: 1 packed sample pairs (default), 0 one sample per lane;
-        None only reads."""
+        """Float-float kernel family: 1 packed sample pairs (default; large products with the table in
+        shared memory), 0 one sample per lane; None only reads."""
         out = ctypes.c_int32()
         check(lib().cgb_op_ff_kernels(self._h.ptr, -1 if variant is None else int(variant), ctypes.byref(out)))
         return int(out.value)

@@ -121,14 +121,18 @@ int cgb_op_lut_grad(cgb_op *op, const double *x, const double *g, double *g_ic, 
  * Voxel shape of the float-float pair kernels: 1 the default (fewest padded samples), 2 a
  * warp per voxel, 0 = timed on the next call (the default at creation); set < 0 only reads.
  * *fwd / *adj (may be NULL) receive the shapes of A and A'.  Results agree to ~1e-16.
- * Setting a shape also keeps this handle on the pair kernels (large products otherwise run
- * with the LUT in shared memory).
+ * Setting a shape also keeps this handle's products on the pair kernels and, with FP32 vectors, on
+ * the gathering or tensor-core ones (large products otherwise run with the LUT in shared
+ * memory), until cgb_op_ff_kernels(op, 1, ...).  Set before the first product, it also forgoes the memory
+ * of the shared-memory products (about 40 bytes per segment at 288 samples).
  */
 int cgb_op_ff_shape(cgb_op *op, int set, int *fwd, int *adj);
 
 /*
  * Float-float kernel family: 1 (default) packed f32x2 pairs of samples on padded LUT rows,
- * 0 one sample per lane; a negative value only reads.  Same arithmetic to ~1e-15.
+ * 0 one sample per lane; a negative value only reads.  Same arithmetic to ~1e-15.  Setting 1
+ * also lets large products run with the LUT in shared memory again after cgb_op_ff_shape or
+ * cgb_op_occupancy kept them from it.
  */
 int cgb_op_ff_kernels(cgb_op *op, int variant, int *out);
 
@@ -347,8 +351,10 @@ int cgb_op_apply_batch(cgb_op *op, int adjoint, int nvec, const void *const *in,
  * set >= 0 stores a choice (0 = tune again on the next call, 1 or 2 = fixed), set < 0 only
  * reads; choice / ms_a / ms_b (may be NULL) receive the choice and the two measured times.
  * Both builds compute the same operations in the same order: results are identical.
- * The float-float slots are those of the pair kernels: setting any choice also keeps this
- * handle on them (large products otherwise run with the LUT in shared memory).
+ * The slots are those of kernels that gather the LUT's rows: setting one also keeps the products of
+ * its kernel (A or A' in its arithmetic) on it, where large ones otherwise run with the LUT in
+ * shared memory, until cgb_op_ff_kernels(op, 1, ...); the solvers' float-float gradient stays on the
+ * pair kernels while any float-float slot is set.
  */
 int cgb_op_occupancy(cgb_op *op, int slot, int set, int *choice, float *ms_a, float *ms_b);
 

@@ -75,3 +75,32 @@ def test_bytes_follow_the_layout():
         assert A.device_bytes() == full
     A.dot(x.float(), arith='f32'), A.T.dot(y.float(), arith='f32')
     assert A.device_bytes() > full
+
+
+def test_set_builds_and_shapes_hold_their_own_products():
+    """A register build that is set keeps the products of its kernel, and no others, from the shared-memory
+    kernels; a shape keeps all; selecting the default family releases both."""
+    from commit_gb300.operator import LinearOperator
+    D, K = _problem(97, 6000)
+    A = LinearOperator(D, K, None)
+    A.tensor_cores(1)
+    x, y = torch.rand(A.nCOLS, dtype=torch.float64, device='cuda'), torch.rand(A.nROWS, dtype=torch.float64, device='cuda')
+    x32, y32 = x.float(), y.float()
+
+    def shared():
+        out = ran(lambda: A.dot(x), 'k_fwd_smem') + ran(lambda: A.T.dot(y), 'k_adj_smem')
+        for ar in ('bf16', 'fp16', 'f32'):
+            out += ran(lambda: A.dot(x32, arith=ar), 'k_fwd_mix_smem') + ran(lambda: A.T.dot(y32, arith=ar), 'k_adj_mix_smem')
+        return out
+    # FP64 A, A'; BF16 A, A'; FP16 A, A'; FP32 A, A'
+    assert shared() == [True] * 8
+    A.occupancy({'bf16_adjoint': 1})
+    assert shared() == [True, True, True, False, True, True, True, True]
+    A.occupancy({'ff_forward': 2, 'f32_forward': 0})
+    assert shared() == [False, True, True, False, True, True, False, True]
+    assert A.ff_kernels(1) == 1
+    assert shared() == [True] * 8
+    A.ff_shape(1)
+    assert shared() == [False] * 8
+    A.ff_kernels(1)
+    assert shared() == [True] * 8
