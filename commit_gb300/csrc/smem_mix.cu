@@ -174,6 +174,10 @@ int mix_plan(cgb_op *op, cudaStream_t st, int arith, int adjoint, MixPlan **out)
     MixPlan shape{};
     if (!mix_shape(op, word, &shape) || (double)op->n * op->nIC < mix_min_items(shape.nc) * op->nV) return CGB_OK;
     if (tc && op->nIC * shape.nc * shape.nq > (adjoint && op->n < kTcAdjDense * op->nV ? 4 : 6)) return CGB_OK;
+    if (op->mixp[f32] && !op->mixp[f32]->img) return CGB_OK;  // there was no room
+    // only now: a product that ends on other kernels prepares the reduced tables itself, and the
+    // preparation waits for the device
+    CGB_TRY(ensure_reduced(op, arith));
     static std::mutex mu;
     std::lock_guard<std::mutex> g(mu);
     if (!op->mixp[f32] || (op->mixp[f32]->img && op->mixp_kind[f32] != arith)) {
@@ -270,7 +274,6 @@ void free_mix_plan(cgb_op *op) {
 
 int forward_smem_mix(cgb_op *op, const float *x, float *y, cudaStream_t st, int arith, int *ran) {
     *ran = 0;
-    CGB_TRY(ensure_reduced(op, arith));
     MixPlan *m;
     CGB_TRY(mix_plan(op, st, arith, 0, &m));
     if (!m) return CGB_OK;
@@ -290,7 +293,6 @@ int forward_smem_mix(cgb_op *op, const float *x, float *y, cudaStream_t st, int 
 
 int adjoint_smem_mix(cgb_op *op, const float *y, double *x, cudaStream_t st, int arith, int *ran) {
     *ran = 0;
-    CGB_TRY(ensure_reduced(op, arith));
     MixPlan *m;
     CGB_TRY(mix_plan(op, st, arith, 1, &m));
     if (!m) return CGB_OK;
