@@ -960,7 +960,7 @@ int build_plan(cgb_op *op, FfPlan *f) {
     if (fs) {
         CGB_TRY(keep_buffer(op, &f->bytes, &f->fimg, (size_t)f->fnc * op->nIC * op->ndirs * f->fcs));
         CGB_TRY(keep_buffer(op, &f->bytes, &f->coef, (size_t)op->nIC * R->nruns));
-        CGB_CUDA(cudaEventCreateWithFlags(&f->done, cudaEventDisableTiming));
+        CGB_TRY(order_create(&f->order));
     }
     if (as) {
         CGB_TRY(keep_buffer(op, &f->bytes, &f->aimg, (size_t)f->anc * f->anb * op->nIC * f->ano * f->acs));
@@ -1040,7 +1040,7 @@ static void drop_plan(cgb_op *op, FfPlan *f) {
     void *p[] = {f->coef, f->fimg, f->colmax, f->aimg, f->run_blk, f->part, f->epart, f->zrow};
     for (void *q : p)
         if (q) cudaFree(q);
-    if (f->done) cudaEventDestroy(f->done);
+    if (f->order.done) cudaEventDestroy(f->order.done);
     op->bytes -= f->bytes;
     memset((void *)f, 0, sizeof(*f));
 }
@@ -1123,7 +1123,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     // the coefficients belong to the handle: a product on another stream waits for the last
     // one (under capture the graph's own order applies)
     const bool cap = capturing(st);
-    if (!cap && f->used && f->last != st) CGB_CUDA(cudaStreamWaitEvent(st, f->done, 0));
+    if (!cap) CGB_TRY(order_enter(&f->order, st));
     if (op->vr1 <= 0 || op->vr0 == 0)
         k_run_coef<<<grid_n((R.nruns + kCoefRuns - 1) / kCoefRuns), 256, 0, st>>>(P, R.run_seg, R.nruns, x, R.eval_ones,
                                                                                   f->coef);
@@ -1140,11 +1140,7 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
         case 6: rc = launch_sm(k_fwd_smem<6>, g, kFwdThreads, smem, st, a); break;
     }
     CGB_TRY(rc);
-    if (!cap) {
-        CGB_CUDA(cudaEventRecord(f->done, st));
-        f->last = st;
-        f->used = 1;
-    }
+    if (!cap) CGB_TRY(order_leave(&f->order, st));
     if (grid) *grid = g;
     *ran = 1;
     return CGB_OK;

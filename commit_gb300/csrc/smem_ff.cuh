@@ -50,6 +50,31 @@ struct RunLayout {
     size_t bytes;                // of the handle's, held here
 };
 
+// Products on different streams take turns with buffers of the handle: each waits for the last one's
+// end, unless that ran on the same stream.  Streams are told apart by their id: the handle of a
+// destroyed stream is given to new ones, and cudaStreamPerThread is one handle for many streams.
+struct StreamOrder {
+    cudaEvent_t done;            // the last product has finished
+    unsigned long long last;     // ... its stream
+    int used;
+};
+inline int order_create(StreamOrder *o) {
+    CGB_CUDA(cudaEventCreateWithFlags(&o->done, cudaEventDisableTiming));
+    return CGB_OK;
+}
+inline int order_enter(const StreamOrder *o, cudaStream_t st) {
+    unsigned long long id = 0;
+    CGB_CUDA(cudaStreamGetId(st, &id));
+    if (o->used && o->last != id) CGB_CUDA(cudaStreamWaitEvent(st, o->done, 0));
+    return CGB_OK;
+}
+inline int order_leave(StreamOrder *o, cudaStream_t st) {
+    CGB_CUDA(cudaEventRecord(o->done, st));
+    CGB_CUDA(cudaStreamGetId(st, &o->last));
+    o->used = 1;
+    return CGB_OK;
+}
+
 // Table images and buffers of the shared-memory float-float products
 struct FfPlan {
     int fwd_ok, adj_ok;          // kernels usable for this handle's shape and table
@@ -67,9 +92,7 @@ struct FfPlan {
     double *part;                // [nIC * nruns][anc] parts of the runs' dot products (anc > 1)
     double *epart;               // [EC and ISO columns][anc]
     double *zrow;                // [nrows] weighted residual (FISTA gradient)
-    cudaEvent_t done;            // the last product that used coef has finished
-    cudaStream_t last;           // ... and its stream
-    int used;
+    StreamOrder order;           // of the products that use coef
     int no_room;                 // the buffers did not fit: not tried again
     size_t bytes;                // of the handle's, held here
 };

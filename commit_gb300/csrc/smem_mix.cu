@@ -139,7 +139,7 @@ int build_mix(cgb_op *op, int word, MixPlan *m) {
     if (m->nc > 1) CGB_TRY(keep_buffer(op, &m->bytes, &m->part, (size_t)runs * m->nc));
     if (m->nc > 1) CGB_TRY(keep_buffer(op, &m->bytes, &m->epart, ((size_t)op->nE * op->nEC + (size_t)op->nISOv * op->nISO) * m->nc));
     CGB_TRY(keep_buffer(op, &m->bytes, &m->img, (size_t)m->nc * op->nIC * op->ndirs * m->cs * word));
-    CGB_CUDA(cudaEventCreateWithFlags(&m->done, cudaEventDisableTiming));
+    CGB_TRY(order_create(&m->order));
     return CGB_OK;
 }
 
@@ -248,25 +248,13 @@ int launch(const cgb_op *op, const MixPlan *m, int arith, int adjoint, const SmM
     return launch_mix_smem_fp16(adjoint, m->nq, g, smem, st, a, m->cs);
 }
 
-// the buffers belong to the handle: a product on another stream waits for the last one
-int enter(MixPlan *m, cudaStream_t st) {
-    if (m->used && m->last != st) CGB_CUDA(cudaStreamWaitEvent(st, m->done, 0));
-    return CGB_OK;
-}
-int leave(MixPlan *m, cudaStream_t st) {
-    CGB_CUDA(cudaEventRecord(m->done, st));
-    m->last = st;
-    m->used = 1;
-    return CGB_OK;
-}
-
 }  // namespace
 
 void free_mix_plan(cgb_op *op) {
     for (MixPlan *&m : op->mixp) {
         if (!m) continue;
         drop(op, m);
-        if (m->done) cudaEventDestroy(m->done);
+        if (m->order.done) cudaEventDestroy(m->order.done);
         delete m;
         m = nullptr;
     }
@@ -281,12 +269,12 @@ int forward_smem_mix(cgb_op *op, const float *x, float *y, cudaStream_t st, int 
     a.x = x;
     a.y = y;
     a.vec_ok = op->nS % 4 == 0 && (uintptr_t)y % 16 == 0;
-    CGB_TRY(enter(m, st));
+    CGB_TRY(order_enter(&m->order, st));
     auto coef = arith == CGB_ARITH_F32 ? k_mix_coef<true> : k_mix_coef<false>;
     coef<<<grid_of((a.nruns + 3) / 4, 8192), 256, 0, st>>>(a, op->seg_f, op->runs->eval_ones ? nullptr : op->eval, op->nF);
     CGB_CUDA(cudaGetLastError());
     CGB_TRY(launch(op, m, arith, 0, a, st));
-    CGB_TRY(leave(m, st));
+    CGB_TRY(order_leave(&m->order, st));
     *ran = 1;
     return CGB_OK;
 }
@@ -296,7 +284,7 @@ int adjoint_smem_mix(cgb_op *op, const float *y, double *x, cudaStream_t st, int
     MixPlan *m;
     CGB_TRY(mix_plan(op, st, arith, 1, &m));
     if (!m) return CGB_OK;
-    CGB_TRY(enter(m, st));
+    CGB_TRY(order_enter(&m->order, st));
     auto pass = [&](cudaStream_t q) -> int {
         SmMixArgs a = mix_args(op, m, arith);
         a.z = y;
@@ -321,7 +309,7 @@ int adjoint_smem_mix(cgb_op *op, const float *y, double *x, cudaStream_t st, int
             },
             [&](int s, cudaStream_t q) { return fibre_sum32_slab(op, op->scratch32, x, s, q); }));
     }
-    CGB_TRY(leave(m, st));
+    CGB_TRY(order_leave(&m->order, st));
     *ran = 1;
     return CGB_OK;
 }

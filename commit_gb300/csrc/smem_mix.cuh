@@ -24,9 +24,7 @@ struct MixPlan {
     float *coef;         // [nIC * nruns]
     float *part;         // [nIC * nruns][nc] (nc > 1)
     double *epart;       // [EC and ISO columns][nc] (nc > 1)
-    cudaEvent_t done;    // the last product has finished with the buffers
-    cudaStream_t last;   // ... and its stream
-    int used;
+    StreamOrder order;   // of the products, which share the buffers
     size_t bytes;        // of the handle's, held here
 };
 

@@ -104,3 +104,29 @@ def test_set_builds_and_shapes_hold_their_own_products():
     assert shared() == [False] * 8
     A.ff_kernels(1)
     assert shared() == [True] * 8
+
+
+def test_products_on_reused_stream_handles():
+    """Streams that come and go: a new stream may have the handle of a destroyed one and is still
+    another stream, so its product waits for the last one before it writes the shared buffers."""
+    from commit_gb300._lib import check, lib, DTYPE_F32, DTYPE_F64
+    from commit_gb300.operator import LinearOperator
+    path = next(l.split()[-1] for l in open('/proc/self/maps') if 'libcudart.so' in l)
+    rt = ctypes.CDLL(path)
+    D, K = _problem(97, 20000, n_mask=9000, dim=(28, 28, 24), ndirs=120)
+    A = LinearOperator(D, K, None)
+    xs = [torch.rand(A.nCOLS, dtype=torch.float64, device='cuda') for _ in range(4)]
+    for dtype, num, arith in ((torch.float64, DTYPE_F64, 1), (torch.float32, DTYPE_F32, 3)):
+        ins = [x.to(dtype) for x in xs]
+        refs = [A.dot(v, arith='fp16' if num == DTYPE_F32 else None) for v in ins]
+        outs = [torch.empty_like(r) for r in refs]
+        torch.cuda.synchronize()
+        for v, out in zip(ins, outs):
+            st = ctypes.c_void_p()
+            assert rt.cudaStreamCreateWithFlags(ctypes.byref(st), 1) == 0    # non-blocking
+            check(lib().cgb_op_apply(A.handle, 0, ctypes.c_void_p(v.data_ptr()), v.numel(), ctypes.c_void_p(out.data_ptr()),
+                                     out.numel(), num, arith, st))
+            assert rt.cudaStreamDestroy(st) == 0                             # its work goes on
+        torch.cuda.synchronize()
+        for out, r in zip(outs, refs):
+            assert torch.equal(out, r)
