@@ -838,7 +838,7 @@ bool fwd_shape(int rows, int nS, FfPlan *f) {
             if (np <= 2) return false;
             continue;
         }
-        if (np * 16 * (nc - 1) >= nS) return false;
+        if (np < 2 || np * 16 * (nc - 1) >= nS) return false;  // no kernel for one pair, no empty last chunk
         f->fnp = np;
         f->fnc = nc;
         f->fcs = 16 * ne;
@@ -1132,7 +1132,6 @@ int forward_smem(cgb_op *op, const double *x, double *y, double *ax, const doubl
     const size_t smem = (size_t)op->nIC * op->ndirs * f->fcs * sizeof(float);
     int rc = CGB_ERR_UNSUPPORTED;
     switch (f->fnp) {
-        case 1: rc = launch_sm(k_fwd_smem<1>, g, kFwdThreads, smem, st, a); break;
         case 2: rc = launch_sm(k_fwd_smem<2>, g, kFwdThreads, smem, st, a); break;
         case 3: rc = launch_sm(k_fwd_smem<3>, g, kFwdThreads, smem, st, a); break;
         case 4: rc = launch_sm(k_fwd_smem<4>, g, kFwdThreads, smem, st, a); break;
