@@ -252,7 +252,10 @@ int launch_chunks(const cgb_op *op, int kind, int rf, const GradStream &S, const
         }
     }
     const int blocks = op->nsm * 8;
-#define CGB_GRAD(I, L, K)                                                                                             if (best == I)                                                                                                        k_grad_chunks<L, K><<<blocks, 256, 0, st>>>(P, kind, rf, S.run_v, S.run_b, S.run_e, S.chunk_beg, S.nchunks, x, g,                                                     partial);
+#define CGB_GRAD(I, L, K)                                                                                        \
+    if (best == I)                                                                                               \
+        k_grad_chunks<L, K><<<blocks, 256, 0, st>>>(P, kind, rf, S.run_v, S.run_b, S.run_e, S.chunk_beg, S.nchunks, \
+                                                    x, g, partial);
     CGB_GRAD(0, 8, 9) CGB_GRAD(1, 8, 12) CGB_GRAD(2, 16, 9) CGB_GRAD(3, 16, 12) CGB_GRAD(4, 32, 9)
 #undef CGB_GRAD
     CGB_CUDA(cudaGetLastError());
