@@ -30,12 +30,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = 'A·x+Aᵀx operator pairs/s (1M-streamline workload)'
 
-# DRAM bytes (read + write) per product, recorded from one ncu capture of this workload
-# (`ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum
-# --clock-control none -k regex:"k_(run_coef|fwd_smem|adj_smem|adj_join|fibre_pass)" --csv python bench.py
-# --steps 1 --warmup 1 --no-e2e --no-cpu`, one pass, full workload).  A constant: the bench
-# line labels it as such.  Keyed by (workload, streamlines, arith); the A entry is the run
-# coefficients and the voxel pass, the A' entry the slabs' voxel, join and fibre passes.
+# DRAM bytes (read + write) per product, recorded once from the hardware counters on this workload.
+# A constant: the bench line labels it as such; a changed kernel does not change it.  Keyed by
+# (workload, streamlines, arith); the A entry is the run coefficients and the voxel pass, the A'
+# entry the slabs' voxel, join and fibre passes.
 MEASURED_TRAFFIC = {('hcp_1m', 1000000, 'ff'): {'forward': 4424852224, 'adjoint': 16377132032}}
 
 
@@ -423,8 +421,8 @@ def run_ours(args):
            'roofline': {'bound': 'hbm', 'kernel': dom, 'achieved': achieved, 'peak': peaks['hbm_gbs'],
                         'unit': 'GB/s', 'frac': achieved / peaks['hbm_gbs'], 'peak_src': peaks['src'],
                         'traffic': traffic_for(args, spec, dom),
-                        'traffic_src': 'recorded constant: dram__bytes_read.sum + dram__bytes_write.sum of one ncu '
-                                       'capture of this workload and arithmetic, per product',
+                        'traffic_src': 'recorded constant: DRAM bytes read + written, from the hardware counters on '
+                                       'this workload and arithmetic, per product',
                         'algorithmic_bytes_per_launch': nbytes,
                         'forward_ms': fwd_ms, 'adjoint_ms': adj_ms,
                         'fma_per_product': nfma, 'achieved_gfma_s': nfma / (dom_ms / 1000.0) / 1e9},
