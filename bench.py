@@ -310,21 +310,17 @@ def workload_config(spec, D, K, args):
             'arith': args.arith, 'l2': 'inputs larger than L2 (y is nV*nS f64), no flush'}
 
 
-def launches_per_pair(A, reduced: bool, tc: bool = False) -> int:
-    """Kernels of one A + A' pair.  FP64 path: the max-|x| pass of the range guard and the
-    forward (large operators: the run coefficients before it), then per adjoint slab a voxel
-    pass (large operators: the join of its parts) and a fibre pass.  Reduced precision: the
-    FP32 -> FP64 column conversion (large operators: the run coefficients) and the forward,
-    the adjoint (slab passes, or the tensor-core voxel pass and its fibre pass) and the
-    FP64 -> FP32 conversion; the tensor-core forward, taken from seven 32-sample blocks x
-    responses on, adds its x*eval pass."""
-    ns = max(1, A.set_slabs(None))
-    if tc and A.ICnRF * -(-A.nSAMPLES // 32) > 6:
-        return 3 + 3
-    if reduced:
-        return 2 + 2 * ns + 1
-    smem = A.ICn * A.ICnRF * A.nSAMPLES >= 1e7 and A.ICn * A.ICnRF >= 4 * -(-A.nSAMPLES // 96) * A.ICnVOX
-    return 3 + 3 * ns if smem else 2 + 2 * ns
+def launches_per_pair(pair) -> tuple:
+    """(kernels of this library that one A + A' pair launches, how they were counted): in a trace of
+    one pair, or the fewest that any pair has (A; the voxel and fibre passes of A')."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    for _ in range(2):  # the first trace of a process starts late
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            pair()
+            torch.cuda.synchronize()
+    n = sum('cgb::' in e.name for e in p.events())
+    return (n, 'traced') if n else (3, 'lower bound, no trace on this machine')
 
 
 def traffic_for(args, spec, dom: str):
@@ -427,7 +423,6 @@ def run_ours(args):
                         'forward_ms': fwd_ms, 'adjoint_ms': adj_ms,
                         'fma_per_product': nfma, 'achieved_gfma_s': nfma / (dom_ms / 1000.0) / 1e9},
            'clocks': clk,
-           'gpu_launches': args.steps * launches_per_pair(A, reduced, reduced and args.arith == 'bf16' and A.tensor_cores()),
            'setup_s': {'generate': tgen, 'create_operator': tcreate},
            'occupancy_tuning': A.occupancy(), 'adjoint_slabs': A.set_slabs(None),
            'tensor_cores': bool(reduced and args.arith == 'bf16' and A.tensor_cores())}
@@ -497,6 +492,8 @@ def run_ours(args):
         cb = cpu_reference(D, K, args.sample_frac, 5, 1, x_full=x.double().cpu().numpy())
         out['parity_vs_reference'] = check_against_reference(A, y, cb, K['wmr'].shape[2], args.arith)
         out['cpu_baseline'] = cb
+    n, how = launches_per_pair(lambda: (A.dot(x, out=y, **kw), At.dot(y, out=g, **kw)))
+    out['gpu_launches'], out['gpu_launches_src'] = args.steps * n, how
     if rank == 0:
         print(json.dumps(out))
     if ws > 1:
