@@ -89,8 +89,8 @@ struct FfPlan {
     int anp, anc, anb, ano, acs;
     float *aimg;                 // [anc][anb][nIC * ano][acs]
     uint32_t *run_blk;           // [anb + 1][nV] first run of the voxel in a range
-    double *part;                // [nIC * nruns][anc] parts of the runs' dot products (anc > 1)
-    double *epart;               // [EC and ISO columns][anc]
+    double *part;                // [nIC * nruns][anc] parts of the runs' dot products
+    double *epart;               // [EC and ISO columns][anc] (anc > 1)
     double *zrow;                // [nrows] weighted residual (FISTA gradient)
     StreamOrder order;           // of the products that use coef
     int no_room;                 // the buffers did not fit: not tried again

@@ -103,7 +103,8 @@ int cgb_op_device_bytes(const cgb_op *op, size_t *bytes);
 
 /*
  * Replace the LUT values (same shapes as at creation; host or device pointers, NULL leaves
- * that compartment unchanged).  Used when the LUT itself is being fitted.  No counterpart
+ * that compartment unchanged).  Complete on return: later products on any stream use the new
+ * values.  Used when the LUT itself is being fitted.  No counterpart
  * in the reference, whose LUTs are fixed after load_kernels (commit/core.pyx:364-433).
  */
 int cgb_op_set_lut(cgb_op *op, const float *lutIC, const float *lutEC, const float *lutISO);
@@ -166,6 +167,9 @@ int cgb_op_set_arith(cgb_op *op, int arith);
  * may have any finite magnitude: the float-float kernels scale operands whose products
  * with the LUT would leave FP32's exponent range by an exact power of two (the forward
  * input as a whole, the adjoint input per voxel row) and scale the results back in FP64.
+ * Under stream capture the product keeps to the kernels that read the handle's tables in place (a
+ * replay follows cgb_op_set_lut); an eager one of a large operator runs on others, and the
+ * two differ in their last bits.
  */
 int cgb_op_apply(cgb_op *op, int adjoint, const void *in, int64_t in_len, void *out, int64_t out_len, int dtype,
                  int arith, void *stream);
