@@ -36,13 +36,18 @@ def _table(D, K, kind):
         w[0, used.argmin(), 40] = 1.0
         y[:] = 0.0
         y[:, 40] = 1.0
+    elif kind.startswith('faint'):               # the same, less extreme: an even table, but uneven dot products
+        w[0, :, 40:42] *= float(kind[5:])
+        w[0, used.argmin(), 40:42] = 1.0
+        y[:, :40] = y[:, 42:] = 0.0
     elif kind == 'zero':                         # rows of zeros
         w[0, ::3] = 0.0
     return dict(K, wmr=w), y
 
 
 @pytest.mark.parametrize('kind,nS,nIC', [('large1e6', 70, 1), ('large1e8', 97, 1), ('small1e6', 97, 1), ('small1e9', 288, 1),
-                                         ('response', 70, 2), ('sample', 97, 1), ('zero', 97, 1)])
+                                         ('response', 70, 2), ('sample', 97, 1), ('faint1e-4', 97, 1), ('faint1e-6', 288, 1),
+                                         ('zero', 97, 1)])
 def test_rows_of_different_size(kind, nS, nIC):
     from commit_gb300.operator import LinearOperator
     D, K = _problem(nS, 6000, nIC=nIC, nEC=0, nISO=0)
